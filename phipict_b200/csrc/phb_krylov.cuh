@@ -1,0 +1,642 @@
+// Device code shared by the Krylov translation units: per-system state, the stencil products on
+// quads, the tile bodies of CG and BiCGStab, the grid barrier and the reductions of the
+// persistent kernels, and the workspace layouts.
+#pragma once
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <initializer_list>
+#include <type_traits>
+#include "phb_device.cuh"
+#include "phb_amg.cuh"
+#include "phb_launch.cuh"
+
+namespace phb {
+
+constexpr int NWARPS = PHB_TILE / 32;
+enum Done : int { RUNNING = 0, CONVERGED = 1, NONFINITE = 2, MAXIT = 3, RISING = 4 };
+constexpr int RISING_CUTOFF = 100;
+
+struct SysState {
+	double tol, rho, alpha, beta, omega, crit, best, last, halfCrit, innerTol;
+	int it, maxit, bestIt, rising, done, restart, saveBest, halfDone, usedIt, innerIts;
+	int launched, pad2;
+};
+static_assert(sizeof(SysState) == 128, "SysState layout");
+
+struct Control {
+	unsigned int counter;
+	int allDone;
+	int loops;
+	int maxLoops;
+	unsigned int barCount; // grid barrier of the persistent solvers: arrival counter
+	int barErr;            // set when a barrier wait ran out (the kernel then returns)
+	int pad[2];
+};
+static_assert(sizeof(Control) == 32, "Control layout");
+
+// device helpers -----------------------------------------------------------------------
+__device__ __forceinline__ double warpSum(double v) {
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+	return v;
+}
+
+__device__ __forceinline__ bool fin(double v) { return isfinite(v); }
+__device__ __forceinline__ double normScale(const int32_t *insts, int inst) { return 1.0 / sqrt(double(insts[inst * PHB_IREC + I_NCELLS])); }
+
+template <int K>
+__device__ __forceinline__ int64_t vk(const int32_t *B, int64_t g, int k) {
+	return g + (int64_t)(K - 1) * B[B_INSTOFF] + (int64_t)k * B[B_INSTN];
+}
+
+template <int D>
+__device__ __forceinline__ void stencilNeighbors(const Dom<double, D> &dom, const Cell &c, int64_t *nb) {
+#pragma unroll
+	for (int f = 0; f < 2 * D; ++f) nb[f] = neighborIndex<double, D>(dom, c, f);
+}
+
+// Krylov tile bodies on quads ------------------------------------------------------------
+// Fields evaluated at the stencil points: at(o) one value, at4(o) four consecutive values.
+// Every multiply-add is an explicit fma, so that the persistent kernel and the per-phase
+// kernels round identically whatever contraction the compiler would choose in each.
+template <typename T>
+struct FX { // a stored vector
+	const T *x;
+	__device__ __forceinline__ T at(int64_t o) const { return x[o]; }
+	__device__ __forceinline__ void at4(int64_t o, int n, bool al, T (&v)[4]) const { ld4(x + o, n, al, v); }
+};
+template <typename T>
+struct FDir { // CG direction p' = z + beta p (z after a restart)
+	const T *z, *p;
+	T beta;
+	bool rs;
+	__device__ __forceinline__ T at(int64_t o) const { return rs ? z[o] : fma(beta, p[o], z[o]); }
+	__device__ __forceinline__ void at4(int64_t o, int n, bool al, T (&v)[4]) const {
+		ld4(z + o, n, al, v);
+		if (rs) return;
+		T b[4];
+		ld4(p + o, n, al, b);
+#pragma unroll
+		for (int i = 0; i < 4; ++i) v[i] = fma(beta, b[i], v[i]);
+	}
+};
+template <typename T>
+struct FBicgP { // BiCGStab direction p = r + beta (p - omega v) (r after a restart)
+	const T *r, *p, *v;
+	T beta, omega;
+	bool rs;
+	__device__ __forceinline__ T at(int64_t o) const { return rs ? r[o] : fma(beta, fma(-omega, v[o], p[o]), r[o]); }
+	__device__ __forceinline__ void at4(int64_t o, int n, bool al, T (&w)[4]) const {
+		ld4(r + o, n, al, w);
+		if (rs) return;
+		T a[4], b[4];
+		ld4(p + o, n, al, a);
+		ld4(v + o, n, al, b);
+#pragma unroll
+		for (int i = 0; i < 4; ++i) w[i] = fma(beta, fma(-omega, b[i], a[i]), w[i]);
+	}
+};
+template <typename T>
+struct FBicgS { // BiCGStab half step s = r - alpha v
+	const T *r, *v;
+	T alpha;
+	__device__ __forceinline__ T at(int64_t o) const { return fma(-alpha, v[o], r[o]); }
+	__device__ __forceinline__ void at4(int64_t o, int n, bool al, T (&w)[4]) const {
+		T b[4];
+		ld4(r + o, n, al, w);
+		ld4(v + o, n, al, b);
+#pragma unroll
+		for (int i = 0; i < 4; ++i) w[i] = fma(-alpha, b[i], w[i]);
+	}
+};
+
+// y = A f and f itself at the quad's cells for every active right-hand side (zeros for the
+// others and past q.n). On the fast path (a quad inside one row whose y and z neighbours are
+// in the block or absent behind a prescribed face) the four cells' stencil rows and neighbour
+// groups are loaded at once, slot by slot; elsewhere every cell resolves its neighbours
+// across faces. The products are summed in the same order on both paths (centre, then faces
+// -x +x -y +y -z +z, a face without neighbour skipped).
+template <typename T, int D, int K, typename F>
+__device__ __forceinline__ void quadApply(const Dom<double, D> &dom, const T *__restrict__ A, const Quad &q, const bool (&act)[K],
+		const F (&fld)[K], T (&y)[K][4], T (&f)[K][4]) {
+	const int64_t N = dom.ncells;
+	if (q.fastW) {
+		// x neighbours of the row ends: across the block's x face when the quad touches it
+		int64_t gW = q.g - 1, gE = q.g + 4;
+		if (q.p[0] == 0 || q.p[0] + 3 == q.B[B_NX] - 1) {
+			Cell c;
+			c.B = q.B;
+			c.p[1] = q.p[1];
+			c.p[2] = q.p[2];
+			if (q.p[0] == 0) {
+				c.p[0] = 0;
+				c.g = (int)q.g;
+				gW = neighborIndex<double, D>(dom, c, 0);
+			}
+			if (q.p[0] + 3 == q.B[B_NX] - 1) {
+				c.p[0] = q.p[0] + 3;
+				c.g = (int)(q.g + 3);
+				gE = neighborIndex<double, D>(dom, c, 1);
+			}
+		}
+		int64_t o[K];
+#pragma unroll
+		for (int k = 0; k < K; ++k) o[k] = vk<K>(q.B, q.g, k);
+		T a[4];
+		ld4(A + q.g, 4, q.al, a);
+#pragma unroll
+		for (int k = 0; k < K; ++k) {
+			if (!act[k]) {
+#pragma unroll
+				for (int i = 0; i < 4; ++i) f[k][i] = 0;
+			} else {
+				fld[k].at4(o[k], 4, q.al, f[k]);
+			}
+#pragma unroll
+			for (int i = 0; i < 4; ++i) y[k][i] = a[i] * f[k][i];
+		}
+		ld4(A + N + q.g, 4, q.al, a);
+#pragma unroll
+		for (int k = 0; k < K; ++k) {
+			if (!act[k]) continue;
+			if (gW >= 0) y[k][0] = fma(a[0], fld[k].at(vk<K>(q.B, gW, k)), y[k][0]);
+#pragma unroll
+			for (int i = 1; i < 4; ++i) y[k][i] = fma(a[i], f[k][i - 1], y[k][i]);
+		}
+		ld4(A + 2 * N + q.g, 4, q.al, a);
+#pragma unroll
+		for (int k = 0; k < K; ++k) {
+			if (!act[k]) continue;
+#pragma unroll
+			for (int i = 0; i < 3; ++i) y[k][i] = fma(a[i], f[k][i + 1], y[k][i]);
+			if (gE >= 0) y[k][3] = fma(a[3], fld[k].at(vk<K>(q.B, gE, k)), y[k][3]);
+		}
+#pragma unroll
+		for (int sl = 3; sl < 2 * D + 1; ++sl) {
+			if ((q.miss >> (sl - 3)) & 1) continue; // behind a prescribed face: no neighbour
+			const int64_t off = sl == 3 ? -(int64_t)q.sy : sl == 4 ? (int64_t)q.sy : sl == 5 ? -(int64_t)q.sz : (int64_t)q.sz;
+			const bool al = sl < 5 ? q.alY : q.alZ;
+			ld4(A + sl * N + q.g, 4, q.al, a);
+#pragma unroll
+			for (int k = 0; k < K; ++k) {
+				if (!act[k]) continue;
+				T v[4];
+				fld[k].at4(o[k] + off, 4, al, v);
+#pragma unroll
+				for (int i = 0; i < 4; ++i) y[k][i] = fma(a[i], v[i], y[k][i]);
+			}
+		}
+		return;
+	}
+#pragma unroll
+	for (int i = 0; i < 4; ++i) {
+#pragma unroll
+		for (int k = 0; k < K; ++k) { y[k][i] = 0; f[k][i] = 0; }
+		if (i >= q.n) continue;
+		Cell c;
+		quadCell<D>(q, i, c);
+		int64_t nb[2 * D];
+		stencilNeighbors<D>(dom, c, nb);
+		const T a0 = A[c.g];
+		T af[2 * D];
+#pragma unroll
+		for (int fc = 0; fc < 2 * D; ++fc) af[fc] = A[(fc + 1) * N + c.g];
+#pragma unroll
+		for (int k = 0; k < K; ++k) {
+			if (!act[k]) continue;
+			const T ci = fld[k].at(vk<K>(c.B, c.g, k));
+			T s = a0 * ci;
+#pragma unroll
+			for (int fc = 0; fc < 2 * D; ++fc)
+				if (nb[fc] >= 0) s = fma(af[fc], fld[k].at(vk<K>(c.B, nb[fc], k)), s);
+			y[k][i] = s;
+			f[k][i] = ci;
+		}
+	}
+}
+
+// r = b - A x per right-hand side, (r, r) and (b, b) into acc[2k], acc[2k+1]; emit(k, o, q,
+// r[4]) stores r.
+template <typename T, int D, int K, typename Emit>
+__device__ __forceinline__ void tileResidual(const Dom<double, D> &dom, const int32_t *sB, int l0, int nc, const T *__restrict__ A,
+		const T *__restrict__ b, const T *__restrict__ x, const bool (&act)[K], double (&acc)[2 * K], Emit emit) {
+	Quad q;
+	quadAt<D, K>(dom.vec4, sB, l0, nc, q);
+	FX<T> fx[K];
+#pragma unroll
+	for (int k = 0; k < K; ++k) fx[k].x = x;
+	T y[K][4], f[K][4];
+	quadApply<T, D, K>(dom, A, q, act, fx, y, f);
+#pragma unroll
+	for (int k = 0; k < K; ++k) {
+		if (!act[k]) continue;
+		const int64_t o = vk<K>(q.B, q.g, k);
+		T bv[4], rv[4];
+		ld4(b + o, q.n, q.al, bv);
+#pragma unroll
+		for (int i = 0; i < 4; ++i) {
+			rv[i] = bv[i] - y[k][i];
+			acc[2 * k] = fma(double(rv[i]), double(rv[i]), acc[2 * k]);
+			acc[2 * k + 1] = fma(double(bv[i]), double(bv[i]), acc[2 * k + 1]);
+		}
+		emit(k, o, q, rv);
+	}
+}
+
+// CG phase 1 on a tile: p' = z + beta p, q = A p', (p', q)
+template <typename T, int D, int K>
+__device__ __forceinline__ void tileCgDirection(const Dom<double, D> &dom, const int32_t *sB, int l0, int nc, const T *__restrict__ A,
+		const T *z, const T *pIn, T *pOut, T *qv, const bool (&act)[K], const bool (&rs)[K], const T (&beta)[K], double (&acc)[K]) {
+	Quad q;
+	quadAt<D, K>(dom.vec4, sB, l0, nc, q);
+	FDir<T> fd[K];
+#pragma unroll
+	for (int k = 0; k < K; ++k) fd[k] = FDir<T>{z, pIn, beta[k], rs[k]};
+	T y[K][4], f[K][4];
+	quadApply<T, D, K>(dom, A, q, act, fd, y, f);
+#pragma unroll
+	for (int k = 0; k < K; ++k) {
+		if (!act[k]) continue;
+		const int64_t o = vk<K>(q.B, q.g, k);
+		st4(pOut + o, q.n, q.al, f[k]);
+		st4(qv + o, q.n, q.al, y[k]);
+#pragma unroll
+		for (int i = 0; i < 4; ++i) acc[k] = fma(double(f[k][i]), double(y[k][i]), acc[k]);
+	}
+}
+
+// CG phase 2 on a tile: x += alpha p, r -= alpha q, (r, r) (xbest = x before, when asked)
+template <typename T, int D, int K>
+__device__ __forceinline__ void tileCgUpdate(const Dom<double, D> &dom, const int32_t *sB, int l0, int nc, T *r, const T *p,
+		const T *qv, T *x, T *xbest, const SysState *sst, double (&acc)[K]) {
+	Quad q;
+	quadAt<D, K>(dom.vec4, sB, l0, nc, q);
+	const int inst = sB[B_INST];
+#pragma unroll
+	for (int k = 0; k < K; ++k) {
+		const SysState &s = sst[inst * K + k];
+		if (s.done != RUNNING) continue;
+		const T alpha = T(s.alpha);
+		const int64_t o = vk<K>(q.B, q.g, k);
+		T xv[4], pv[4], rv[4], qq[4];
+		ld4(x + o, q.n, q.al, xv);
+		ld4(p + o, q.n, q.al, pv);
+		ld4(r + o, q.n, q.al, rv);
+		ld4(qv + o, q.n, q.al, qq);
+		if (s.saveBest && xbest) st4(xbest + o, q.n, q.al, xv);
+#pragma unroll
+		for (int i = 0; i < 4; ++i) {
+			xv[i] = fma(alpha, pv[i], xv[i]);
+			rv[i] = fma(-alpha, qq[i], rv[i]);
+			acc[k] = fma(double(rv[i]), double(rv[i]), acc[k]);
+		}
+		st4(x + o, q.n, q.al, xv);
+		st4(r + o, q.n, q.al, rv);
+	}
+}
+
+// BiCGStab phase 1 on a tile: p = r + beta (p - omega v), v = A p, (r0, v)
+template <typename T, int D, int K>
+__device__ __forceinline__ void tileBicgV(const Dom<double, D> &dom, const int32_t *sB, int l0, int nc, const T *__restrict__ A,
+		const T *r, const T *pIn, const T *vIn, T *pOut, T *vOut, const T *r0, const bool (&act)[K], const bool (&rs)[K],
+		const T (&beta)[K], const T (&omega)[K], double (&acc)[K]) {
+	Quad q;
+	quadAt<D, K>(dom.vec4, sB, l0, nc, q);
+	FBicgP<T> fp[K];
+#pragma unroll
+	for (int k = 0; k < K; ++k) fp[k] = FBicgP<T>{r, pIn, vIn, beta[k], omega[k], rs[k]};
+	T y[K][4], f[K][4];
+	quadApply<T, D, K>(dom, A, q, act, fp, y, f);
+#pragma unroll
+	for (int k = 0; k < K; ++k) {
+		if (!act[k]) continue;
+		const int64_t o = vk<K>(q.B, q.g, k);
+		st4(pOut + o, q.n, q.al, f[k]);
+		st4(vOut + o, q.n, q.al, y[k]);
+		T r0v[4];
+		ld4(r0 + o, q.n, q.al, r0v);
+#pragma unroll
+		for (int i = 0; i < 4; ++i) acc[k] = fma(double(r0v[i]), double(y[k][i]), acc[k]);
+	}
+}
+
+// BiCGStab phase 2 on a tile: s = r - alpha v, t = A s, (t, s), (t, t), (s, s)
+template <typename T, int D, int K>
+__device__ __forceinline__ void tileBicgT(const Dom<double, D> &dom, const int32_t *sB, int l0, int nc, const T *__restrict__ A,
+		const T *r, const T *v, T *t, const bool (&act)[K], const T (&alpha)[K], double (&acc)[3 * K]) {
+	Quad q;
+	quadAt<D, K>(dom.vec4, sB, l0, nc, q);
+	FBicgS<T> fs[K];
+#pragma unroll
+	for (int k = 0; k < K; ++k) fs[k] = FBicgS<T>{r, v, alpha[k]};
+	T y[K][4], f[K][4];
+	quadApply<T, D, K>(dom, A, q, act, fs, y, f);
+#pragma unroll
+	for (int k = 0; k < K; ++k) {
+		if (!act[k]) continue;
+		const int64_t o = vk<K>(q.B, q.g, k);
+		st4(t + o, q.n, q.al, y[k]);
+#pragma unroll
+		for (int i = 0; i < 4; ++i) {
+			acc[3 * k + 0] = fma(double(y[k][i]), double(f[k][i]), acc[3 * k + 0]);
+			acc[3 * k + 1] = fma(double(y[k][i]), double(y[k][i]), acc[3 * k + 1]);
+			acc[3 * k + 2] = fma(double(f[k][i]), double(f[k][i]), acc[3 * k + 2]);
+		}
+	}
+}
+
+// BiCGStab phase 3 on a tile: x += alpha p + omega s, r = s - omega t, (r0, r), (r, r); after
+// a converged half step x += alpha p, r = s
+template <typename T, int D, int K>
+__device__ __forceinline__ void tileBicgUpdate(const Dom<double, D> &dom, const int32_t *sB, int l0, int nc, T *r, const T *r0,
+		const T *p, const T *v, const T *t, T *x, const SysState *sst, double (&acc)[2 * K]) {
+	Quad q;
+	quadAt<D, K>(dom.vec4, sB, l0, nc, q);
+	const int inst = sB[B_INST];
+#pragma unroll
+	for (int k = 0; k < K; ++k) {
+		const SysState &s = sst[inst * K + k];
+		if (s.done != RUNNING) continue;
+		const T alpha = T(s.alpha), omega = T(s.omega);
+		const int64_t o = vk<K>(q.B, q.g, k);
+		T rv[4], vv[4], pv[4], xv[4];
+		ld4(r + o, q.n, q.al, rv);
+		ld4(v + o, q.n, q.al, vv);
+		ld4(p + o, q.n, q.al, pv);
+		ld4(x + o, q.n, q.al, xv);
+		if (s.halfDone) {
+#pragma unroll
+			for (int i = 0; i < 4; ++i) {
+				xv[i] = fma(alpha, pv[i], xv[i]);
+				rv[i] = fma(-alpha, vv[i], rv[i]);
+			}
+		} else {
+			T tv[4], r0v[4];
+			ld4(t + o, q.n, q.al, tv);
+			ld4(r0 + o, q.n, q.al, r0v);
+#pragma unroll
+			for (int i = 0; i < 4; ++i) {
+				const T si = fma(-alpha, vv[i], rv[i]);
+				xv[i] = fma(omega, si, fma(alpha, pv[i], xv[i]));
+				rv[i] = fma(-omega, tv[i], si);
+				acc[2 * k + 0] = fma(double(r0v[i]), double(rv[i]), acc[2 * k + 0]);
+				acc[2 * k + 1] = fma(double(rv[i]), double(rv[i]), acc[2 * k + 1]);
+			}
+		}
+		st4(x + o, q.n, q.al, xv);
+		st4(r + o, q.n, q.al, rv);
+	}
+}
+
+// SolverTolerance._resolve_scale (solvers/tolerance.py:241-257)
+__device__ __forceinline__ double resolveTol(const phb_tolerance &t, double scale) {
+	double tol = 0.0;
+	if (t.rtol > 0) tol = t.rtol * scale;
+	if (t.atol > 0) tol = fmax(tol, t.atol);
+	tol = fmax(tol, t.floor_eps * scale);
+	if (!(tol > 0.0)) tol = t.fallback;
+	return tol;
+}
+
+// rho/beta of a running system from the new (r, z) (the preconditioned CG of
+// amg_pcg_solve, solvers/amg.py:1544): the first iteration after a restart takes rho only.
+__device__ __forceinline__ void pcgRho(SysState &s, double rz) {
+	if (s.restart) s.rho = rz;
+	else {
+		s.beta = rz / s.rho;
+		s.rho = rz;
+		if (!fin(s.beta)) s.done = NONFINITE;
+	}
+	if (!fin(rz)) s.done = NONFINITE;
+}
+
+// persistent solvers ---------------------------------------------------------------------
+// One cooperative launch runs a whole solve. The CTAs are co-resident (cooperative launch)
+// and meet at grid barriers instead of kernel boundaries, so an iteration costs a few
+// barrier round trips instead of kernel launches and the vectors stay in L2. Every barrier
+// wait is bounded: when it runs out it sets Control::barErr and every CTA leaves the kernel
+// (phb_solve_results then reports every system non-finite; inside a refinement the unfinished
+// inner solve leaves the outer loop unconverged). Each CTA keeps its own copy of the per-system
+// scalars in shared memory and reduces the per-tile partials itself, in the same fixed order
+// as every other CTA, so all CTAs take the same decisions without broadcasting them.
+constexpr unsigned int BARRIER_SPIN_LIMIT = 1u << 24;
+constexpr unsigned int BARRIER_ERR_POLL = 1023; // spins between reads of Control::barErr
+
+// Sense-reversing arrival counter: CTA 0 adds 2^31 - (gridDim.x - 1), every other CTA adds 1,
+// so the counter's top bit flips exactly when the last CTA of a generation arrives and the
+// low bits return to where they were (no reset, no second atomic). The arrival is a release
+// and the poll an acquire at GPU scope; with the CTA barriers on both sides that orders every
+// thread's writes before the barrier against every thread's reads after it. A CTA that has
+// seen the flip does not read barErr: a CTA that gave up at this barrier had arrived at it
+// (arrival comes before the wait), so the flip proves the phase complete, and the next
+// barrier, where that CTA never arrives, ends everyone else's wait through barErr.
+__device__ __forceinline__ unsigned int barrierArrive(unsigned int *count, unsigned int add) {
+	unsigned int old;
+	asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(count), "r"(add) : "memory");
+	return old;
+}
+
+__device__ __forceinline__ unsigned int barrierPoll(const unsigned int *count) {
+	unsigned int v;
+	asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+	return v;
+}
+
+__device__ __forceinline__ bool gridBarrier(Control *ctrl, unsigned int spinLimit = BARRIER_SPIN_LIMIT) {
+	__shared__ int sOk;
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		const unsigned int add = blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1) : 1u;
+		const unsigned int old = barrierArrive(&ctrl->barCount, add);
+		int ok = 1;
+		for (unsigned int spins = 1; ((barrierPoll(&ctrl->barCount) ^ old) & 0x80000000u) == 0; ++spins) {
+			if ((spins & BARRIER_ERR_POLL) == 0 && (spins > spinLimit || *(volatile int *)&ctrl->barErr)) {
+				atomicExch(&ctrl->barErr, 1);
+				ok = 0;
+				break;
+			}
+			__nanosleep(32);
+		}
+		sOk = ok;
+	}
+	__syncthreads();
+	return sOk;
+}
+
+// Block sum of NV values written to dst[0..NV) by the first threads.
+template <int NV>
+__device__ __forceinline__ void blockSumTo(double (&v)[NV], double *dst) {
+	__shared__ double sm[NV][NWARPS];
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+	for (int q = 0; q < NV; ++q) {
+		const double s = warpSum(v[q]);
+		if (lane == 0) sm[q][warp] = s;
+	}
+	__syncthreads();
+	if (threadIdx.x < NV) {
+		double s = 0;
+#pragma unroll
+		for (int w = 0; w < NWARPS; ++w) s += sm[threadIdx.x][w];
+		dst[threadIdx.x] = s;
+	}
+	__syncthreads();
+}
+
+// Visit this CTA's tiles with the block record staged in sB.
+template <int D, typename F>
+__device__ __forceinline__ void forMyTiles(const Dom<double, D> &dom, int32_t *sB, F f) {
+	int staged = -1; // the block whose record sB holds (uniform over the CTA)
+	for (int tile = blockIdx.x; tile < dom.ntiles; tile += gridDim.x) {
+		const int b = __ldg(dom.tiles + 2 * tile);
+		const int l0 = __ldg(dom.tiles + 2 * tile + 1);
+		if (b != staged) {
+			__syncthreads();
+			if (threadIdx.x < PHB_BREC) sB[threadIdx.x] = __ldg(dom.blocks + b * PHB_BREC + threadIdx.x);
+			__syncthreads();
+			staged = b;
+		}
+		const int nc = sB[B_NX] * sB[B_NY] * (D > 2 ? sB[B_NZ] : 1);
+		f(tile, l0, nc);
+	}
+}
+
+// All CTAs: reduce every running system's partials (the group scheme of finalizeSystems) and
+// update the CTA's state copy; returns the number of systems still running.
+template <int K, int NQ, int INSTQ = -1, typename Fn>
+__device__ __forceinline__ int reduceStates(const int32_t *insts, int ninst, const double *partial, SysState *sst, Fn fn) {
+	constexpr int NV = NQ + 1;
+	__shared__ int running;
+	__shared__ double gsm[NWARPS][NV];
+	if (threadIdx.x == 0) running = 0;
+	__syncthreads();
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int nsys = ninst * K;
+	int G = NWARPS;
+	while (G > 1 && G * nsys > NWARPS) G >>= 1;
+	const int NG = NWARPS / G;
+	const int group = warp / G, wg = warp - group * G;
+	for (int base = 0; base < nsys; base += NG) {
+		const int s = base + group;
+		const bool act = s < nsys && sst[s].done == RUNNING;
+		double a0[NV], a1[NV];
+#pragma unroll
+		for (int q = 0; q < NV; ++q) { a0[q] = 0; a1[q] = 0; }
+		if (act) {
+			const int inst = s / K, k = s - inst * K;
+			const int t0 = insts[inst * PHB_IREC + I_TILESTART], tc = insts[inst * PHB_IREC + I_TILECOUNT];
+			const int stride = G * 32;
+			auto load = [&](int t, double *a) {
+				const double *pp = partial + (size_t)(t0 + t) * K * NQ;
+#pragma unroll
+				for (int q = 0; q < NQ; ++q) a[q] += __ldcg(pp + k * NQ + q);
+				if (INSTQ >= 0) {
+#pragma unroll
+					for (int kk = 0; kk < K; ++kk) a[NQ] += __ldcg(pp + kk * NQ + (INSTQ < 0 ? 0 : INSTQ));
+				}
+			};
+			int t = wg * 32 + lane;
+			for (; t + stride < tc; t += 2 * stride) { load(t, a0); load(t + stride, a1); }
+			if (t < tc) load(t, a0);
+		}
+#pragma unroll
+		for (int q = 0; q < NV; ++q) {
+			const double v = warpSum(a0[q] + a1[q]);
+			if (lane == 0) gsm[warp][q] = v;
+		}
+		__syncthreads();
+		if (act && wg == 0 && lane == 0) {
+			double red[NV];
+#pragma unroll
+			for (int q = 0; q < NV; ++q) {
+				double v = 0;
+				for (int w = 0; w < G; ++w) v += gsm[group * G + w][q];
+				red[q] = v;
+			}
+			fn(sst[s], s / K, red, red[NQ]);
+		}
+		if (wg == 0 && lane == 0 && s < nsys && sst[s].done == RUNNING) atomicAdd(&running, 1);
+		__syncthreads();
+	}
+	const int r = running;
+	__syncthreads();
+	return r;
+}
+
+// The reference stop rule of the first residual (kResidual) applied to a CTA state copy.
+template <int K, bool BICG, bool STOPSTART>
+__device__ __forceinline__ void residualDecision(const Dom<double, 3> *, SysState &s, double ns, const double *red, double bb,
+		const phb_tolerance &tol) {
+	if (tol.mode == 1) s.tol = resolveTol(tol, sqrt(bb / double(K)) * ns);
+	const double crit = sqrt(red[0]) * ns;
+	s.rho = red[0];
+	s.restart = 1;
+	s.crit = crit;
+	if (!fin(crit)) { s.done = NONFINITE; s.usedIt = 0; }
+	else if ((BICG || STOPSTART) ? crit < s.tol : crit == 0.0) { s.done = CONVERGED; s.usedIt = BICG ? -1 : 0; }
+}
+
+// host side --------------------------------------------------------------------------------
+inline size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
+
+// Dom::vec4 of a launch: every operand on a 16-byte boundary and a cell count that keeps the
+// stencil's slot rows aligned
+inline int vec4Ok(const phb_domain *dom, std::initializer_list<const void *> ptrs) {
+	if (dom->ncells % 4) return 0;
+	for (const void *p : ptrs)
+		if (p && ((uintptr_t)p & 15)) return 0;
+	return 1;
+}
+
+struct Layout {
+	size_t off[12];
+	size_t total;
+};
+
+inline int vecCount(int kind) { return kind == 0 ? 5 : 7; } // CG: r q p0 p1 xbest; BiCG: r r0 p0 p1 v0 v1 t
+
+inline Layout solveLayout(const phb_domain *dom, int kind, int vecBytes, int nrhs) {
+	Layout L;
+	size_t o = 0;
+	const size_t vb = align256((size_t)dom->ncells * nrhs * vecBytes);
+	for (int i = 0; i < vecCount(kind); ++i) { L.off[i] = o; o += vb; }
+	L.off[10] = o; // partials: two halves of up to 3 values per tile and right-hand side
+	o += align256((size_t)dom->ntiles * nrhs * 3 * 2 * sizeof(double));
+	L.total = o;
+	return L;
+}
+
+struct StateLayout { size_t ctrl, st, ctrl2, st2, total; };
+inline StateLayout stateLayout(const phb_domain *dom, int nrhs) {
+	StateLayout L;
+	const size_t nsys = (size_t)dom->ninst * nrhs;
+	L.ctrl = 0;
+	L.st = 256;
+	L.ctrl2 = align256(L.st + nsys * sizeof(SysState));
+	L.st2 = L.ctrl2 + 256;
+	L.total = align256(L.st2 + nsys * sizeof(SysState));
+	return L;
+}
+
+inline int numSMs() {
+	static int cache[64] = {0};
+	int dev = 0;
+	if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+	if (!cache[dev]) {
+		int v = 0;
+		if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
+		cache[dev] = v;
+	}
+	return cache[dev];
+}
+
+// kInit launched on `s`: the initial state of the nsys systems of a solve (krylov.cu)
+int launchInit(SysState *st, int nsys, const phb_tolerance &tol, int fromInner, int maxit, Control *ctrl, cudaStream_t s);
+
+// A persistent solve recorded on `s` (persistent.cu).
+template <typename T, int D, int K>
+int launchPersistent(const phb_domain *dom, const phb_solve *sv, cudaStream_t s, bool stopStart, int fromInner);
+
+} // namespace phb
