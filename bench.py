@@ -422,7 +422,7 @@ def run_ours(args, rank, world, local):
                   "limited_by": ("grid-barrier and L2 latency: the ~60 MB working set stays in L2 (DRAM traffic "
                                  "is ~1.5 % of the algorithmic bytes), so the fraction of HBM peak is low by "
                                  "construction; HBM-bound fractions are measured by the roofline sweep") if amg else None,
-                  "kernel": ("persistent PCG iteration (V-cycle + direction + update, kCgPersistent)" if amg
+                  "kernel": ("persistent PCG iteration (V-cycle + direction + update, kPcg)" if amg
                              else "CG iteration (kCgDirection + kCgUpdate)"),
                   "achieved": round(achieved, 1) if achieved else None, "peak": pk.get("hbm_gbs"),
                   "unit": "GB/s", "frac": round(achieved / pk["hbm_gbs"], 4) if achieved else None,

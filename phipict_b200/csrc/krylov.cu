@@ -1208,7 +1208,7 @@ static int noAllocScratch(cudaStream_t s, void **out) {
 template <typename T, int D, int K>
 static int runCgNoAlloc(const phb_domain *dom, const phb_solve *sv, phb_solve_result *out, cudaStream_t s) {
 	Dom<double, D> dm(*dom);
-	const Layout L = solveLayout(dom, 0, sizeof(T), K);
+	const Layout L = solveLayout(dom, 0, sizeof(T), K, true);
 	const StateLayout SL = stateLayout(dom, K);
 	char *w = (char *)sv->work;
 	char *sb = (char *)sv->state;
@@ -1272,7 +1272,7 @@ static int runCgNoAlloc(const phb_domain *dom, const phb_solve *sv, phb_solve_re
 extern "C" int64_t phb_cg_noalloc_bytes(const phb_domain *dom, int dtype, int nrhs) {
 	if (!dom) return -1;
 	const int vb = dtype == PHB_F64 ? 8 : 4;
-	return (int64_t)(solveLayout(dom, 0, vb, nrhs).total + stateLayout(dom, nrhs).total);
+	return (int64_t)(solveLayout(dom, 0, vb, nrhs, true).total + stateLayout(dom, nrhs).total);
 }
 
 extern "C" int phb_cg_solve_noalloc(const phb_domain *dom, int dtype, int nrhs, const void *A, const void *b, void *x,
@@ -1318,7 +1318,7 @@ extern "C" int phb_cg_solve_noalloc(const phb_domain *dom, int dtype, int nrhs, 
 	sv.b = b;
 	sv.x = x;
 	sv.work = scratch;
-	sv.state = (char *)scratch + solveLayout(dom, 0, dtype == PHB_F64 ? 8 : 4, nrhs).total;
+	sv.state = (char *)scratch + solveLayout(dom, 0, dtype == PHB_F64 ? 8 : 4, nrhs, true).total;
 	cudaStream_t st = (cudaStream_t)stream;
 	PHB_SOLVE_DISPATCH(dom->dims, dtype, nrhs, return runCgNoAlloc<T, D, KK>(dom, &sv, out, st));
 	return PHB_OK;

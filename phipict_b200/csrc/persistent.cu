@@ -1,24 +1,15 @@
-// The persistent Krylov solvers: one cooperative launch runs a whole CG, multigrid-preconditioned
-// CG or BiCGStab solve, with grid barriers between its phases (phb_krylov.cuh).
+// The persistent Krylov solvers: one cooperative launch runs a whole CG or BiCGStab solve, with
+// grid barriers between its phases (phb_krylov.cuh). The multigrid-preconditioned CG is in pcg.cu.
 #include "phb_krylov.cuh"
 
 namespace phb {
 
-// PC: AMG-preconditioned CG (float, one right-hand side): every iteration first runs the
-// V-cycle of `mg` on r, level by level between grid barriers, and takes the direction from z.
-// QUADS (kCgPersistentQuads, for a finest level of at least AMG_QUAD_MIN_CELLS cells): the
-// finest restriction and prolongation in their one-coarse-cell-per-thread and quad forms. It is
-// a kernel of its own, so that the smaller grids' kernel keeps the compiler's register choice,
-// and is held to four resident CTAs per SM (64 registers, some spills), which measured faster
-// on large grids than the 128 registers the compiler takes at two CTAs per SM.
-template <typename T, int D, int K, bool STOPSTART, bool PC, bool QUADS>
+template <typename T, int D, int K, bool STOPSTART>
 __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, const T *__restrict__ A, const T *__restrict__ b,
 		T *__restrict__ x, T *__restrict__ r, T *__restrict__ p0, T *__restrict__ p1, T *__restrict__ q, T *__restrict__ xbest,
-		SysState *st, double *partial, Control *ctrl, const phb_tolerance &tol, int returnBest, int maxit, const AmgView<D> &mg) {
-	static_assert(!PC || (std::is_same<T, float>::value && K == 1), "the V-cycle preconditions float single-rhs CG");
+		SysState *st, double *partial, Control *ctrl, const phb_tolerance &tol, int returnBest, int maxit) {
 	extern __shared__ SysState sst[];
 	__shared__ int32_t sB[PHB_BREC];
-	__shared__ int32_t sBs[PC ? 4 : 1][PHB_BREC];
 	const int nsys = dom.ninst * K;
 	for (int s = threadIdx.x; s < nsys; s += blockDim.x) sst[s] = st[s];
 	__syncthreads();
@@ -47,44 +38,8 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 		residualDecision<K, false, STOPSTART>(nullptr, s, normScale(dom.insts, in), red, bb, tol);
 	});
 	T *pIn = p0, *pOut = p1;
-	// the direction is built from z = M r when preconditioned, from r otherwise
-	const T *dsrc = r;
-	if constexpr (PC) dsrc = (const T *)mg.x[0];
 	for (int iter = 0; running > 0 && iter <= maxit + 1; ++iter) {
-		if constexpr (PC) {
-			const int L = mg.nlevels;
-			constexpr bool quads = QUADS;
-			for (int l = 0; l + 1 < L; ++l) {
-				if (l == 0 && quads) {
-					for (int sub = blockIdx.x; sub < mg.lv[1].ntiles * RESTRICT1_PER_TILE; sub += gridDim.x) amgRestrictCoarseCell<D>(mg, 0, sub, sB);
-				} else {
-					// up to four of this CTA's sub-tiles per pass, their loads in flight together
-					const int nsub = mg.lv[l + 1].ntiles * Restrict<D>::PER_TILE;
-					for (int sub = blockIdx.x; sub < nsub; sub += 4 * gridDim.x)
-						amgRestrictMulti<D, 4>(mg, l, sub, gridDim.x, nsub, sBs);
-				}
-				if (!gridBarrier(ctrl)) return;
-			}
-			amgCoarseRows<D>(mg, int(blockIdx.x * NWARPS + (threadIdx.x >> 5)), int(gridDim.x * NWARPS));
-			if (!gridBarrier(ctrl)) return;
-			for (int l = L - 2; l >= 1; --l) {
-				for (int sub = blockIdx.x; sub < mg.lv[l].ntiles * AMG_SUBTILES; sub += gridDim.x) {
-					const int q = sub % AMG_SUBTILES;
-					amgProlongTile<D>(mg, l, sub / AMG_SUBTILES, sB, mg.x[l], q, q + 1);
-				}
-				if (!gridBarrier(ctrl)) return;
-			}
-			pp = partial + (size_t)(ph++ & 1) * half;
-			for (int tile = blockIdx.x; tile < dom.ntiles; tile += gridDim.x) {
-				// the finest level on quads: with the wall rows on the vector path it beats the
-				// per-cell form on every grid measured (the 442,368-cell duct: 18.5 -> 16.7 ms/step)
-				double acc[1] = {amgProlongQuad<D>(mg, 0, tile, sB, mg.x[0])};
-				blockSumTo<1>(acc, pp + tile);
-			}
-			if (!gridBarrier(ctrl)) return;
-			reduceStates<1, 1>(dom.insts, dom.ninst, pp, sst, [&](SysState &s, int, const double *red, double) { pcgRho(s, red[0]); });
-		}
-		// p' = z + beta p (z = r without preconditioner), q = A p', (p', q)
+		// p' = r + beta p, q = A p', (p', q)
 		pp = partial + (size_t)(ph++ & 1) * half;
 		forMyTiles<D>(dom, sB, [&](int tile, int l0, int nc) {
 			const int inst = sB[B_INST];
@@ -100,7 +55,7 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 			double acc[K];
 #pragma unroll
 			for (int k = 0; k < K; ++k) acc[k] = 0;
-			tileCgDirection<T, D, K>(dom, sB, l0, nc, A, dsrc, pIn, pOut, q, act, rs, beta, acc);
+			tileCgDirection<T, D, K>(dom, sB, l0, nc, A, r, pIn, pOut, q, act, rs, beta, acc);
 			blockSumTo<K>(acc, pp + (size_t)tile * K);
 		});
 		if (!gridBarrier(ctrl)) return;
@@ -135,7 +90,7 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 			if (crit < s.tol) s.done = CONVERGED;
 			else if (s.it >= s.maxit) s.done = MAXIT;
 			else if (returnBest && s.rising >= RISING_CUTOFF) s.done = RISING;
-			else if (!PC) {
+			else {
 				s.beta = red[0] / s.rho;
 				s.rho = red[0];
 				if (!fin(s.beta)) s.done = NONFINITE;
@@ -167,29 +122,20 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 	}
 }
 
-// Resident CTAs per SM that the register budget must allow. The preconditioned solve keeps
-// at least three (at most 85 registers): a grid of one CTA per 1024-cell tile then stays
-// co-resident up to 444 tiles (the 442,368-cell duct has 432). The plain float32 CG is bound
+// Resident CTAs per SM that the register budget must allow. The plain float32 CG is bound
 // by HBM on large grids and is faster with more warps in flight: four CTAs in 3D (64
 // registers), five in 2D (48), which it fits without spilling. Several right-hand sides and
 // float64 need more registers per thread.
-template <typename T, int D, int K, bool PC>
+template <typename T, int D, int K>
 constexpr int cgMinBlocks() {
-	return PC ? 3 : (std::is_same<T, float>::value && K == 1) ? (D == 2 ? 5 : 4) : (K == 1 ? 3 : 2);
-}
-
-template <typename T, int D, int K, bool STOPSTART, bool PC = false>
-__global__ void __launch_bounds__(PHB_TILE, (cgMinBlocks<T, D, K, PC>())) kCgPersistent(Dom<double, D> dom, const T *__restrict__ A, const T *__restrict__ b,
-		T *__restrict__ x, T *__restrict__ r, T *__restrict__ p0, T *__restrict__ p1, T *__restrict__ q, T *__restrict__ xbest,
-		SysState *st, double *partial, Control *ctrl, phb_tolerance tol, int returnBest, int maxit, AmgView<D> mg) {
-	cgPersistentBody<T, D, K, STOPSTART, PC, false>(dom, A, b, x, r, p0, p1, q, xbest, st, partial, ctrl, tol, returnBest, maxit, mg);
+	return (std::is_same<T, float>::value && K == 1) ? (D == 2 ? 5 : 4) : (K == 1 ? 3 : 2);
 }
 
 template <typename T, int D, int K, bool STOPSTART>
-__global__ void __launch_bounds__(PHB_TILE, 4) kCgPersistentQuads(Dom<double, D> dom, const T *__restrict__ A, const T *__restrict__ b,
+__global__ void __launch_bounds__(PHB_TILE, (cgMinBlocks<T, D, K>())) kCgPersistent(Dom<double, D> dom, const T *__restrict__ A, const T *__restrict__ b,
 		T *__restrict__ x, T *__restrict__ r, T *__restrict__ p0, T *__restrict__ p1, T *__restrict__ q, T *__restrict__ xbest,
-		SysState *st, double *partial, Control *ctrl, phb_tolerance tol, int returnBest, int maxit, AmgView<D> mg) {
-	cgPersistentBody<T, D, K, STOPSTART, true, true>(dom, A, b, x, r, p0, p1, q, xbest, st, partial, ctrl, tol, returnBest, maxit, mg);
+		SysState *st, double *partial, Control *ctrl, phb_tolerance tol, int returnBest, int maxit) {
+	cgPersistentBody<T, D, K, STOPSTART>(dom, A, b, x, r, p0, p1, q, xbest, st, partial, ctrl, tol, returnBest, maxit);
 }
 
 template <typename T, int D, int K>
@@ -324,6 +270,9 @@ __global__ void __launch_bounds__(PHB_TILE) kBicgPersistent(Dom<double, D> dom, 
 // sized so that every CTA is resident; the launch fails rather than deadlocks otherwise).
 template <typename T, int D, int K>
 int launchPersistent(const phb_domain *dom, const phb_solve *sv, cudaStream_t s, bool stopStart, int fromInner) {
+	if constexpr (std::is_same<T, float>::value && K == 1) {
+		if (sv->amg && sv->kind == 0) return launchPcg<D>(dom, sv, s, stopStart, fromInner);
+	}
 	Dom<double, D> dm(*dom);
 	const Layout L = solveLayout(dom, sv->kind, sizeof(T), K);
 	const StateLayout SL = stateLayout(dom, K);
@@ -361,20 +310,11 @@ int launchPersistent(const phb_domain *dom, const phb_solve *sv, cudaStream_t s,
 	if (sv->kind == 0) {
 		T *r = (T *)(w + L.off[0]), *q = (T *)(w + L.off[1]), *p0 = (T *)(w + L.off[2]), *p1 = (T *)(w + L.off[3]);
 		T *xbest = sv->return_best ? (T *)(w + L.off[4]) : nullptr;
-		AmgView<D> mg = {};
 		auto launch = [&](auto kern) -> int {
 			cfg.gridDim = dim3(grid((const void *)kern));
-			PHB_CUDA(cudaLaunchKernelEx(&cfg, kern, dm, A, b, x, r, p0, p1, q, xbest, st, partial, ctrl, sv->tol, sv->return_best, maxit, mg));
+			PHB_CUDA(cudaLaunchKernelEx(&cfg, kern, dm, A, b, x, r, p0, p1, q, xbest, st, partial, ctrl, sv->tol, sv->return_best, maxit));
 			return PHB_OK;
 		};
-		if constexpr (std::is_same<T, float>::value && K == 1) {
-			if (sv->amg) {
-				mg = makeAmgView<D>(*sv->amg, (const float *)r, sv->amg->levels[0].x);
-				if (amgFineQuads(mg))
-					return stopStart ? launch(kCgPersistentQuads<T, D, K, true>) : launch(kCgPersistentQuads<T, D, K, false>);
-				return stopStart ? launch(kCgPersistent<T, D, K, true, true>) : launch(kCgPersistent<T, D, K, false, true>);
-			}
-		}
 		return stopStart ? launch(kCgPersistent<T, D, K, true>) : launch(kCgPersistent<T, D, K, false>);
 	}
 	T *r = (T *)(w + L.off[0]), *r0 = (T *)(w + L.off[1]), *p0 = (T *)(w + L.off[2]), *p1 = (T *)(w + L.off[3]);

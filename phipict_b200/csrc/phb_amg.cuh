@@ -68,10 +68,12 @@ __host__ inline AmgView<D> makeAmgView(const phb_amg &a, const float *r, float *
 	return v;
 }
 
-// The finest level of a large grid (bandwidth-bound: several tiles per resident CTA) runs its
-// restriction one coarse cell per thread and its prolongation on quads, which move the same
-// bytes with far fewer instructions; a smaller grid is bound by latency and keeps the
-// per-cell forms, which spread the work over more threads. Both give the same bits.
+// Per-level kernels of the cycle (the graph and host solver modes and phb_amg_vcycle; the
+// persistent solver has its own phases, pcg.cu). The finest level of a large grid
+// (bandwidth-bound: several tiles per resident CTA) runs its restriction one coarse cell per
+// thread and its prolongation on quads, which move the same bytes with far fewer instructions;
+// a smaller grid is bound by latency and keeps the per-cell forms, which spread the work over
+// more threads. Both give the same bits.
 constexpr int64_t AMG_QUAD_MIN_CELLS = 1 << 20;
 template <int D>
 __host__ __device__ __forceinline__ bool amgFineQuads(const AmgView<D> &mg) { return mg.lv[0].ncells >= AMG_QUAD_MIN_CELLS; }
@@ -333,85 +335,8 @@ __device__ __forceinline__ int restrictParts(int l0, int nc) {
 	return (cells + Restrict<D>::CELLS - 1) / Restrict<D>::CELLS;
 }
 
-// Restriction of up to NS sub-tiles sub0, sub0 + stride, ... (< nsub) of level l+1 at once:
-// their block records staged together into sBs, every thread's fine residuals evaluated for
-// all of them before the shuffle trees and stores, so that their loads overlap. Same
-// arithmetic and summation order as amgRestrictPart.
-template <int D, int NS>
-__device__ __forceinline__ void amgRestrictMulti(const AmgView<D> &mg, int l, int sub0, int stride, int nsub,
-		int32_t (*sBs)[PHB_BREC]) {
-	using R = Restrict<D>;
-	const Dom<float, D> &fd = mg.lv[l], &cd = mg.lv[l + 1];
-	const float *A = mg.A[l];
-	const float *wd = mg.wd[l];
-	const float *b = mg.b[l];
-	float *bc = mg.b[l + 1];
-	int bi[NS], l0[NS], part[NS];
-	__syncthreads();
-#pragma unroll
-	for (int s = 0; s < NS; ++s) {
-		const int sub = sub0 + s * stride;
-		bi[s] = -1;
-		if (sub < nsub) {
-			const int tile = sub / R::PER_TILE;
-			part[s] = sub - tile * R::PER_TILE;
-			bi[s] = __ldg(cd.tiles + 2 * tile);
-			l0[s] = __ldg(cd.tiles + 2 * tile + 1);
-			if (threadIdx.x < PHB_BREC) sBs[s][threadIdx.x] = __ldg(cd.blocks + bi[s] * PHB_BREC + threadIdx.x);
-		}
-	}
-	__syncthreads();
-	const int o = int(threadIdx.x) % R::G; // fine cell of its aggregate
-	float v[NS];
-	bool store[NS];
-#pragma unroll
-	for (int s = 0; s < NS; ++s) {
-		v[s] = 0.f;
-		store[s] = false;
-		if (bi[s] < 0) continue;
-		const int32_t *sB = sBs[s];
-		const int nc = sB[B_NX] * sB[B_NY] * (D > 2 ? sB[B_NZ] : 1);
-		if (part[s] >= restrictParts<D>(l0[s], nc)) continue;
-		const int lc = l0[s] + part[s] * R::CELLS + int(threadIdx.x) / R::G;
-		if (!(lc < nc && lc < l0[s] + PHB_TILE_CELLS)) continue;
-		store[s] = o == 0;
-		const int32_t *FB = fd.blk(bi[s]);
-		const int nx = sB[B_NX], ny = sB[B_NY];
-		const int cp[3] = {lc % nx, (lc / nx) % ny, D > 2 ? lc / (nx * ny) : 0};
-		Cell c;
-		bool fvalid = true;
-#pragma unroll
-		for (int a = 0; a < 3; ++a) {
-			const int fs = __ldg(FB + B_NX + a);
-			const int oa = (o >> a) & 1;
-			const bool co = a < D && sB[B_NX + a] < fs;
-			c.p[a] = co ? 2 * cp[a] + oa : cp[a];
-			fvalid &= co ? c.p[a] < fs : oa == 0;
-		}
-		if (fvalid) {
-			c.B = FB;
-			c.b = bi[s];
-			c.g = __ldg(FB + B_CELLOFF) + flat(FB, c.p);
-			c.mi = c.g;
-			v[s] = amgFineResidual<D>(fd, A, wd, b, c);
-		}
-	}
-#pragma unroll
-	for (int s = 0; s < NS; ++s) {
-#pragma unroll
-		for (int m = 1; m < R::G; m <<= 1) v[s] += __shfl_xor_sync(0xffffffffu, v[s], m);
-	}
-#pragma unroll
-	for (int s = 0; s < NS; ++s) {
-		if (!store[s]) continue;
-		const int lc = l0[s] + part[s] * R::CELLS + int(threadIdx.x) / R::G;
-		bc[sBs[s][B_CELLOFF] + lc] = v[s];
-	}
-}
-
 // Restriction for coarse sub-tile `sub` (part sub % PER_TILE of tile sub / PER_TILE) of level
-// l+1: b_{l+1} = P^T (b_l - A_l omega D^-1 b_l). Level vectors are read with plain loads: in
-// the persistent solver other CTAs wrote them earlier in the same launch.
+// l+1: b_{l+1} = P^T (b_l - A_l omega D^-1 b_l).
 template <int D>
 __device__ __forceinline__ void amgRestrictSub(const AmgView<D> &mg, int l, int sub, int32_t *sB) {
 	const Dom<float, D> &cd = mg.lv[l + 1];

@@ -595,15 +595,25 @@ struct Layout {
 	size_t total;
 };
 
-inline int vecCount(int kind) { return kind == 0 ? 5 : 7; } // CG: r q p0 p1 xbest; BiCG: r r0 p0 p1 v0 v1 t
+// CG: r q p0 p1 xbest, and the second residual of the preconditioned CG (float, one right-hand
+// side); BiCG: r r0 p0 p1 v0 v1 t
+inline int vecCount(int kind, bool pcg) { return kind == 0 ? (pcg ? 6 : 5) : 7; }
 
-inline Layout solveLayout(const phb_domain *dom, int kind, int vecBytes, int nrhs) {
+// partials per tile of the preconditioned CG: its finest restriction has at most 16 items per
+// coarse tile, and no level has more tiles than the finest
+constexpr int PCG_PARTIALS = 16;
+
+// plain: the layout of a solve that is never preconditioned
+inline Layout solveLayout(const phb_domain *dom, int kind, int vecBytes, int nrhs, bool plain = false) {
 	Layout L;
 	size_t o = 0;
+	const bool pcg = !plain && kind == 0 && vecBytes == 4 && nrhs == 1;
 	const size_t vb = align256((size_t)dom->ncells * nrhs * vecBytes);
-	for (int i = 0; i < vecCount(kind); ++i) { L.off[i] = o; o += vb; }
+	for (int i = 0; i < vecCount(kind, pcg); ++i) { L.off[i] = o; o += vb; }
+	L.off[9] = o; // block tables of all levels (PcgBlock, pcg.cu)
+	if (pcg) o += align256((size_t)dom->nblocks * PHB_AMG_MAX_LEVELS * 128);
 	L.off[10] = o; // partials: two halves of up to 3 values per tile and right-hand side
-	o += align256((size_t)dom->ntiles * nrhs * 3 * 2 * sizeof(double));
+	o += align256((size_t)dom->ntiles * (pcg ? PCG_PARTIALS : nrhs * 3) * 2 * sizeof(double));
 	L.total = o;
 	return L;
 }
@@ -634,6 +644,10 @@ inline int numSMs() {
 
 // kInit launched on `s`: the initial state of the nsys systems of a solve (krylov.cu)
 int launchInit(SysState *st, int nsys, const phb_tolerance &tol, int fromInner, int maxit, Control *ctrl, cudaStream_t s);
+
+// A persistent preconditioned CG recorded on `s` (pcg.cu).
+template <int D>
+int launchPcg(const phb_domain *dom, const phb_solve *sv, cudaStream_t s, bool stopStart, int fromInner);
 
 // A persistent solve recorded on `s` (persistent.cu).
 template <typename T, int D, int K>
