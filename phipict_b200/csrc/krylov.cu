@@ -136,24 +136,10 @@ __device__ __forceinline__ void setLoop(const LoopCond lc, Control *ctrl) {
 }
 
 // kernels ------------------------------------------------------------------------------
-// Initial state of every system. fromInner: the tolerance was written into
-// SysState::innerTol by the refinement residual (mode ignored).
+// Initial state of every system and a fresh control block.
 __global__ void kInit(SysState *st, int nsys, phb_tolerance tol, int fromInner, int maxit, Control *ctrl, int maxLoops) {
 	for (int s = threadIdx.x; s < nsys; s += blockDim.x) {
-		double t;
-		if (fromInner) t = st[s].innerTol;
-		else if (tol.mode == 0) t = tol.atol;
-		else if (tol.mode == 2) t = tol.values[s];
-		else t = NAN; // resolved from the right-hand side by kResidual
-		SysState z;
-		memset(&z, 0, sizeof(z));
-		z.tol = t;
-		z.innerTol = t;
-		z.maxit = maxit;
-		z.best = INFINITY;
-		z.restart = 1;
-		z.bestIt = -1;
-		st[s] = z;
+		st[s] = initialState(tol, s, fromInner ? st[s].innerTol : 0.0, fromInner, maxit);
 	}
 	if (threadIdx.x == 0) {
 		ctrl->counter = 0; ctrl->allDone = 0; ctrl->loops = 0; ctrl->maxLoops = maxLoops;

@@ -29,7 +29,6 @@
 namespace phb {
 
 constexpr int PCG_ITEMS = 8; // work items per phase that a CTA keeps in shared memory
-constexpr size_t PCG_REC_MAX = 48 * 1024; // block tables of all levels kept in shared memory up to this size
 // Four fine cells per lane in the restriction from this many fine cells on (below, two: the
 // coarse levels have too few rows to fill the chip)
 constexpr int64_t PCG_WIDE_MIN = 1 << 17;
@@ -37,64 +36,13 @@ constexpr int64_t PCG_WIDE_MIN = 1 << 17;
 // Below this many tiles (two per SM) the finest prolongation and direction take quarter tiles
 constexpr int PCG_QUARTER_TILES = 296;
 
-// What the phases need of one block of one level. The cell across a face that is not fixed is an
-// affine function of the position (periodic: the other end of the row; connected: phiPICT's axis
-// mapping): map[f] = c0 + cx x + cy y + cz z. The coarse cell across a face is the same map of
-// the next level at the coarse position (a connection that reverses an axis has even sizes).
-struct __align__(16) PcgBlock {
-	int nx, ny, nz, off;
-	int inst, ncells;
-	unsigned int open; // bit f: face f is not fixed
-	unsigned int al;   // rows of four may be loaded as vectors here and across every open face
-	int4 map[6];
-};
-static_assert(sizeof(PcgBlock) == 128, "PcgBlock layout");
-
-template <int D>
-__device__ __forceinline__ void pcgBuildBlock(const int32_t *blocks, int b, PcgBlock &o) {
-	const int32_t *B = blocks + b * PHB_BREC;
-	const int n[3] = {B[B_NX], B[B_NY], D > 2 ? B[B_NZ] : 1};
-	o.nx = n[0]; o.ny = n[1]; o.nz = n[2];
-	o.off = B[B_CELLOFF];
-	o.inst = B[B_INST];
-	o.ncells = n[0] * n[1] * n[2];
-	unsigned int open = 0;
-	bool al = ((n[0] | o.off) & 3) == 0;
-	for (int f = 0; f < 6; ++f) {
-		int4 m = make_int4(0, 0, 0, 0);
-		if (f < 2 * D && fType(B, f) != FT_FIXED) {
-			open |= 1u << f;
-			Dom<float, D> d;
-			d.blocks = blocks;
-			// the map from its values at the corner (0, 0, 0) of the face and one step along each
-			// tangential axis (the position along the face's own axis does not matter)
-			int v[4];
-			for (int k = 0; k < 4; ++k) {
-				Cell c;
-				c.B = B;
-				c.p[0] = c.p[1] = c.p[2] = 0;
-				c.p[f >> 1] = (f & 1) ? n[f >> 1] - 1 : 0;
-				if (k && k - 1 != (f >> 1) && n[k - 1] > 1) c.p[k - 1] = 1;
-				c.g = 0; c.mi = 0;
-				v[k] = (int)neighbor<float, D>(d, c, f).g;
-			}
-			m = make_int4(v[0], v[1] - v[0], v[2] - v[0], v[3] - v[0]);
-			if (f >= 2) al = al && m.y == 1 && ((m.x | m.z | m.w) & 3) == 0;
-		}
-		o.map[f] = m;
-	}
-	o.open = open;
-	o.al = al;
-}
 // the same tables in global memory, for domains with too many blocks for shared memory
 template <int D>
-__global__ void kPcgBlocks(AmgView<D> mg, PcgBlock *out) {
+__global__ void kPcgTabs(AmgView<D> mg, BlockTab *out) {
 	const int nblk = mg.lv[0].nblocks;
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nblk * mg.nlevels; i += gridDim.x * blockDim.x)
-		pcgBuildBlock<D>(mg.lv[i / nblk].blocks, i % nblk, out[i]);
+		buildBlockTab<D>(mg.lv[i / nblk].blocks, i % nblk, out[i]);
 }
-__device__ __forceinline__ int pcgMap(const int4 &m, int x, int y, int z) { return m.x + m.y * x + m.z * y + m.w * z; }
-
 template <int D>
 struct PcgArgs {
 	Dom<double, D> dom;
@@ -106,7 +54,7 @@ struct PcgArgs {
 	int64_t half; // doubles per half of the partials
 	Control *ctrl;
 	phb_tolerance tol;
-	const PcgBlock *blocks; // tables in global memory, or null: built in shared memory
+	const BlockTab *blocks; // tables in global memory, or null: built in shared memory
 	int returnBest, maxit, stopStart, quarter;
 	unsigned int vec; // bit l: the operands of level l start on 16-byte boundaries
 };
@@ -124,32 +72,6 @@ __device__ __forceinline__ void ld4f(const float *p, float (&v)[4]) {
 	v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
 }
 __device__ __forceinline__ void st4f(float *p, const float (&v)[4]) { *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]); }
-
-// Indices of the neighbours of cell g (x, y, z), or of four cells of an aligned row from g on
-// (W >= 4: the +x neighbour is that of the last one, the y and z neighbours start rows of four).
-// A face without neighbour gets g itself and no bit in `has`: every load is issued without a
-// branch, and what it brings is left out of the sum.
-template <int D, int W>
-__device__ __forceinline__ unsigned int pcgNeighbors(const PcgBlock &B, int g, int x, int y, int z, int (&o)[2 * D]) {
-	unsigned int has = (1u << (2 * D)) - 1;
-	const int sy = B.nx, sz = B.nx * B.ny;
-	o[0] = g - 1; o[1] = g + W; o[2] = g - sy; o[3] = g + sy;
-	if constexpr (D > 2) { o[4] = g - sz; o[5] = g + sz; }
-	bool end[2 * D];
-	end[0] = x == 0; end[1] = x + W == B.nx; end[2] = y == 0; end[3] = y + 1 == B.ny;
-	if constexpr (D > 2) { end[4] = z == 0; end[5] = z + 1 == B.nz; }
-#pragma unroll
-	for (int f = 0; f < 2 * D; ++f)
-		if (end[f]) {
-			if ((B.open >> f) & 1) {
-				o[f] = pcgMap(B.map[f], x, y, z);
-			} else {
-				o[f] = g;
-				has &= ~(1u << f);
-			}
-		}
-	return has;
-}
 
 // the finest field of the restriction: r' = r - alpha q (UPD) or r, and s = omega/D r'
 template <bool UPD>
@@ -210,9 +132,9 @@ __device__ __forceinline__ void stRow(float *p, int cnt, const float (&v)[V]) {
 // t = r' - A omega D^-1 r' is stored for the way up, the aggregate sums (x pairs, then y, then z:
 // a fixed order) go to bc. UPD: also x += alpha p, r' stored, (r', r') returned. All loads are
 // issued before the first product (a face that is resolved by a branch of its own costs its own
-// round trip to L2). V = 4: rows of four as vectors (PcgBlock::al); V = 2: any rows.
+// round trip to L2). V = 4: rows of four as vectors (BlockTab::rows4); V = 2: any rows.
 template <int D, int V, bool UPD>
-__device__ __forceinline__ double pcgRestrictItem(const PcgBlock &B, const PcgBlock &CB, int first, int64_t N,
+__device__ __forceinline__ double pcgRestrictItem(const BlockTab &B, const BlockTab &CB, int first, int64_t N,
 		const float *__restrict__ A, const PcgFine<UPD> f, float *__restrict__ t, float *__restrict__ bc,
 		float *__restrict__ rOut, float *__restrict__ x, const float *__restrict__ p, float *xbest) {
 	constexpr int R = PcgRows<D>::R, H = V / 2;
@@ -221,7 +143,7 @@ __device__ __forceinline__ double pcgRestrictItem(const PcgBlock &B, const PcgBl
 	const int cnx = CB.nx, cny = CB.ny;
 	const bool kx = cnx < fnx, ky = cny < fny, kz = D > 2 && CB.nz < fnz;
 	const int lc = first + grp * H;
-	const bool valid = lc < CB.ncells;
+	const bool valid = lc < CB.cells();
 	const int crow = lc / cnx;
 	const int cx = lc - crow * cnx;
 	const int cz = D > 2 ? crow / cny : 0;
@@ -252,15 +174,15 @@ __device__ __forceinline__ double pcgRestrictItem(const PcgBlock &B, const PcgBl
 		// aggregate is one row thin there
 		int ow = g - 1, oe = g + cnt;
 		bool hw = true, he = true;
-		if (x0 == 0) { hw = B.open & 1; ow = hw ? pcgMap(B.map[0], x0, y, z) : g; }
-		if (x0 + cnt == fnx) { he = (B.open >> 1) & 1; oe = he ? pcgMap(B.map[1], x0 + cnt - 1, y, z) : g; }
+		if (x0 == 0) { hw = B.open(0); ow = hw ? tabMap(B.map[0], x0, y, z) : g; }
+		if (x0 + cnt == fnx) { he = B.open(1); oe = he ? tabMap(B.map[1], x0 + cnt - 1, y, z) : g; }
 		auto outside = [&](int fc, bool atEnd, int off, int &o, int &st, bool &has) {
 			o = g + off;
 			st = 1;
 			has = true;
 			if (atEnd) {
-				has = (B.open >> fc) & 1;
-				o = has ? pcgMap(B.map[fc], x0, y, z) : g;
+				has = B.open(fc);
+				o = has ? tabMap(B.map[fc], x0, y, z) : g;
 				st = has ? B.map[fc].y : 1;
 			}
 		};
@@ -346,7 +268,7 @@ __device__ __forceinline__ double pcgRestrictItem(const PcgBlock &B, const PcgBl
 // z at one cell of a level: s + e + omega/D (t - A P e) with s = omega/D b, e the coarse correction
 // of its aggregate
 template <int D>
-__device__ __forceinline__ float pcgProlongCell(const PcgBlock &B, const PcgBlock &CB, int g, int x, int y, int z, int64_t N,
+__device__ __forceinline__ float pcgProlongCell(const BlockTab &B, const BlockTab &CB, int g, int x, int y, int z, int64_t N,
 		const float *__restrict__ A, const float *__restrict__ wd, float bv, float tv, const float *__restrict__ e) {
 	const int kx = CB.nx < B.nx, ky = CB.ny < B.ny, kz = D > 2 ? CB.nz < B.nz : 0;
 	const int cx = x >> kx, cy = y >> ky, cz = z >> kz;
@@ -369,8 +291,8 @@ __device__ __forceinline__ float pcgProlongCell(const PcgBlock &B, const PcgBloc
 #pragma unroll
 	for (int f = 0; f < 2 * D; ++f)
 		if (end[f]) {
-			if ((B.open >> f) & 1) {
-				o[f] = pcgMap(CB.map[f], cx, cy, cz);
+			if (B.open(f)) {
+				o[f] = tabMap(CB.map[f], cx, cy, cz);
 			} else {
 				o[f] = ce;
 				has &= ~(1u << f);
@@ -391,7 +313,7 @@ __device__ __forceinline__ float pcgProlongCell(const PcgBlock &B, const PcgBloc
 
 // The same for four cells of an aligned row (its x size is a multiple of four, so it is halved)
 template <int D>
-__device__ __forceinline__ void pcgProlongQuad(const PcgBlock &B, const PcgBlock &CB, int g, int x, int y, int z, int64_t N,
+__device__ __forceinline__ void pcgProlongQuad(const BlockTab &B, const BlockTab &CB, int g, int x, int y, int z, int64_t N,
 		const float *__restrict__ A, const float *__restrict__ wd, const float (&bv)[4], const float (&tv)[4],
 		const float *__restrict__ e, float (&out)[4]) {
 	const int ky = CB.ny < B.ny, kz = D > 2 ? CB.nz < B.nz : 0;
@@ -415,8 +337,8 @@ __device__ __forceinline__ void pcgProlongQuad(const PcgBlock &B, const PcgBlock
 	for (int f = 0; f < 2 * D; ++f) {
 		st[f] = 1;
 		if (end[f]) {
-			if ((B.open >> f) & 1) {
-				o[f] = pcgMap(CB.map[f], f == 1 ? cx + 1 : cx, cy, cz);
+			if (B.open(f)) {
+				o[f] = tabMap(CB.map[f], f == 1 ? cx + 1 : cx, cy, cz);
 				st[f] = CB.map[f].y;
 			} else {
 				o[f] = ce;
@@ -451,10 +373,10 @@ __device__ __forceinline__ void pcgProlongQuad(const PcgBlock &B, const PcgBlock
 
 // y = A f at one cell and f there (fields of phb_krylov.cuh) ...
 template <int D, typename F>
-__device__ __forceinline__ float pcgCellApply(const PcgBlock &B, int g, int x, int y, int z, int64_t N, const float *__restrict__ A,
+__device__ __forceinline__ float pcgCellApply(const BlockTab &B, int g, int x, int y, int z, int64_t N, const float *__restrict__ A,
 		const F &f, float &fc) {
 	int o[2 * D];
-	const unsigned int has = pcgNeighbors<D, 1>(B, g, x, y, z, o);
+	const unsigned int has = tabNeighbors<D, 1>(B, g, x, y, z, o);
 	float a[2 * D + 1], v[2 * D];
 	fc = f.at(g);
 #pragma unroll
@@ -468,12 +390,12 @@ __device__ __forceinline__ float pcgCellApply(const PcgBlock &B, int g, int x, i
 }
 // ... and at four cells of an aligned row
 template <int D, typename F>
-__device__ __forceinline__ void pcgQuadApply(const PcgBlock &B, int g, int x, int y, int z, int64_t N, const float *__restrict__ A,
+__device__ __forceinline__ void pcgQuadApply(const BlockTab &B, int g, int x, int y, int z, int64_t N, const float *__restrict__ A,
 		const F &f, float (&yv)[4], float (&fc)[4]) {
 	int o[2 * D];
-	const unsigned int has = pcgNeighbors<D, 4>(B, g, x, y, z, o);
+	const unsigned int has = tabNeighbors<D, 4>(B, g, x, y, z, o);
 	// the +x neighbour across a block face is that of the row's last cell
-	if (x + 4 == B.nx && (has & 2)) o[1] = pcgMap(B.map[1], x + 3, y, z);
+	if (x + 4 == B.nx && (has & 2)) o[1] = tabMap(B.map[1], x + 3, y, z);
 	float a[4], v[2 * D - 2][4];
 	f.at4(g, 4, true, fc);
 	float w = f.at(o[0]), e = f.at(o[1]);
@@ -501,97 +423,10 @@ __device__ __forceinline__ void pcgQuadApply(const PcgBlock &B, int g, int x, in
 
 // a restriction without update, of either width
 template <int D>
-__device__ __forceinline__ void pcgRestrictItemAny(bool w4, const PcgBlock &B, const PcgBlock &CB, int first, int64_t N,
+__device__ __forceinline__ void pcgRestrictItemAny(bool w4, const BlockTab &B, const BlockTab &CB, int first, int64_t N,
 		const float *__restrict__ A, const PcgFine<false> f, float *__restrict__ t, float *__restrict__ bc) {
 	if (w4) pcgRestrictItem<D, 4, false>(B, CB, first, N, A, f, t, bc, nullptr, nullptr, nullptr, nullptr);
 	else pcgRestrictItem<D, 2, false>(B, CB, first, N, A, f, t, bc, nullptr, nullptr, nullptr, nullptr);
-}
-
-// Every CTA reduces the partials of every running system (items range(inst) = first, count) and
-// updates its own copy of the states: all the warps on one system when there are few, a warp per
-// system (four in flight) when there are many. Returns the systems still running.
-template <int NQ, typename Range, typename Fn>
-__device__ __forceinline__ int pcgReduce(int ninst, const double *pp, SysState *sst, Range range, Fn fn) {
-	__shared__ int running;
-	__shared__ double gsm[NWARPS][NQ];
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	if (threadIdx.x == 0) running = 0;
-	if (ninst >= NWARPS) {
-		constexpr int U = 4;
-		__syncthreads();
-		int mine = 0;
-		for (int s0 = warp; s0 < ninst; s0 += U * NWARPS) {
-			double a[U][NQ];
-			bool act[U];
-#pragma unroll
-			for (int u = 0; u < U; ++u) {
-				const int s = s0 + u * NWARPS;
-				act[u] = s < ninst && sst[s].done == RUNNING;
-#pragma unroll
-				for (int q = 0; q < NQ; ++q) a[u][q] = 0;
-				if (!act[u]) continue;
-				const int2 rg = range(s);
-				for (int t = lane; t < rg.y; t += 32)
-#pragma unroll
-					for (int q = 0; q < NQ; ++q) a[u][q] += __ldcg(pp + (size_t)(rg.x + t) * NQ + q);
-			}
-#pragma unroll
-			for (int u = 0; u < U; ++u) {
-#pragma unroll
-				for (int q = 0; q < NQ; ++q) a[u][q] = warpSum(a[u][q]);
-				if (act[u] && lane == u) fn(sst[s0 + u * NWARPS], s0 + u * NWARPS, a[u]);
-			}
-			if (lane < U) {
-				const int s = s0 + lane * NWARPS;
-				if (s < ninst && sst[s].done == RUNNING) ++mine;
-			}
-		}
-		if (mine) atomicAdd(&running, mine);
-		__syncthreads();
-		return running;
-	}
-	int G = NWARPS;
-	while (G > 1 && G * ninst > NWARPS) G >>= 1;
-	const int s = warp / G, wg = warp - s * G;
-	const bool act = s < ninst && sst[s].done == RUNNING;
-	double a0[NQ], a1[NQ];
-#pragma unroll
-	for (int q = 0; q < NQ; ++q) a0[q] = a1[q] = 0;
-	if (act) {
-		const int2 rg = range(s);
-		const int stride = G * 32;
-		int t = wg * 32 + lane;
-		for (; t + stride < rg.y; t += 2 * stride)
-#pragma unroll
-			for (int q = 0; q < NQ; ++q) {
-				a0[q] += __ldcg(pp + (size_t)(rg.x + t) * NQ + q);
-				a1[q] += __ldcg(pp + (size_t)(rg.x + t + stride) * NQ + q);
-			}
-		if (t < rg.y)
-#pragma unroll
-			for (int q = 0; q < NQ; ++q) a0[q] += __ldcg(pp + (size_t)(rg.x + t) * NQ + q);
-	}
-#pragma unroll
-	for (int q = 0; q < NQ; ++q) {
-		const double v = warpSum(a0[q] + a1[q]);
-		if (lane == 0) gsm[warp][q] = v;
-	}
-	__syncthreads();
-	if (s < ninst && wg == 0 && lane == 0) {
-		if (act) {
-			double red[NQ];
-#pragma unroll
-			for (int q = 0; q < NQ; ++q) {
-				double v = 0;
-				for (int w = 0; w < G; ++w) v += gsm[warp + w][q];
-				red[q] = v;
-			}
-			fn(sst[s], s, red);
-		}
-		if (sst[s].done == RUNNING) atomicAdd(&running, 1);
-	}
-	__syncthreads();
-	return running;
 }
 
 // The dense operator of the last level, a warp per row, finished instances left out
@@ -629,19 +464,19 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 	const int nblk = a.dom.nblocks;
 	const int T = a.mg.nlevels - 1;
 	const unsigned int grid = gridDim.x;
-	PcgBlock *sBlk = reinterpret_cast<PcgBlock *>(sst + ninst);
+	BlockTab *sBlk = reinterpret_cast<BlockTab *>(sst + ninst);
 	if (threadIdx.x == 0) sAl = a.vec;
 	for (int s = threadIdx.x; s < ninst; s += blockDim.x) sst[s] = a.st[s];
 	if (!a.blocks)
-		for (int i = threadIdx.x; i < (T + 1) * nblk; i += blockDim.x) pcgBuildBlock<D>(a.mg.lv[i / nblk].blocks, i % nblk, sBlk[i]);
+		for (int i = threadIdx.x; i < (T + 1) * nblk; i += blockDim.x) buildBlockTab<D>(a.mg.lv[i / nblk].blocks, i % nblk, sBlk[i]);
 	__syncthreads();
-	const PcgBlock *blks = a.blocks ? a.blocks : sBlk;
+	const BlockTab *blks = a.blocks ? a.blocks : sBlk;
 	// rows of four only where every block of the level allows them
 	for (int i = threadIdx.x; i < (T + 1) * nblk; i += blockDim.x)
-		if (!blks[i].al) atomicAnd(&sAl, ~(1u << (i / nblk)));
+		if (!blks[i].rows4()) atomicAnd(&sAl, ~(1u << (i / nblk)));
 	__syncthreads();
 	const unsigned int alMask = sAl;
-	auto blocksOf = [&](int l) -> const PcgBlock * { return blks + l * nblk; };
+	auto blocksOf = [&](int l) -> const BlockTab * { return blks + l * nblk; };
 	auto wide = [&](int l) -> bool { return ((alMask >> l) & 1) && a.mg.lv[l].ncells >= PCG_WIDE_MIN; };
 	auto perR = [&](int l) -> int { return wide(l) ? PcgItem<D, 4>::PER : PcgItem<D, 2>::PER; };
 	// Finest level outside the restriction: whole tiles (rows of four, or four cells per thread
@@ -675,7 +510,7 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 		}
 	};
 	const int64_t N = a.dom.ncells;
-	const PcgBlock *blk0 = blocksOf(0);
+	const BlockTab *blk0 = blocksOf(0);
 	const bool al0 = (alMask & 1) && !quarter;
 	const int perA = perR(0);
 	const int n0 = a.dom.ntiles * per0;
@@ -690,15 +525,15 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 		const int32_t *in = a.mg.lv[1].insts + inst * PHB_IREC;
 		return make_int2(__ldg(in + I_TILESTART) * perA, __ldg(in + I_TILECOUNT) * perA);
 	};
-	auto quad = [&](const PcgBlock &B, int l0, auto f) {
+	auto quad = [&](const BlockTab &B, int l0, auto f) {
 		const int l = l0 + 4 * int(threadIdx.x);
-		if (l >= B.ncells) return;
+		if (l >= B.cells()) return;
 		const int row = l / B.nx, z = D > 2 ? row / B.ny : 0;
 		f(B.off + l, l - row * B.nx, row - z * B.ny, z);
 	};
 	// cells 256 apart (loads of a warp stay contiguous whatever the row length), two at a time
-	auto cells = [&](const PcgBlock &B, int l0, auto f) {
-		const int end = min(B.ncells, l0 + cells0);
+	auto cells = [&](const BlockTab &B, int l0, auto f) {
+		const int end = min(B.cells(), l0 + cells0);
 		for (int l = l0 + int(threadIdx.x); l < end; l += 2 * PHB_TILE) {
 			int g[2], x[2], y[2], z[2];
 			const int n = l + PHB_TILE < end ? 2 : 1;
@@ -718,7 +553,7 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 	// r = b - A x, (r, r), (b, b)
 	nextPartials();
 	visit(1, a.dom.tiles, n0, per0, cells0, [&](int it, int b, int l0) {
-		const PcgBlock &B = blk0[b];
+		const BlockTab &B = blk0[b];
 		if (sst[B.inst].done != RUNNING) return;
 		double acc[2] = {0, 0};
 		const FX<float> fx{a.x};
@@ -755,7 +590,7 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 		blockSumTo<2>(acc, pp + (size_t)it * 2);
 	});
 	if (!gridBarrier(a.ctrl)) return;
-	int running = pcgReduce<2>(ninst, pp, sst, tileRange, [&](SysState &s, int in, const double *red) {
+	int running = reduceSystems<1, 2, -1>(ninst, pp, sst, tileRange, [&](SysState &s, int in, const double *red, double) {
 		if (a.stopStart) residualDecision<1, false, true>(nullptr, s, normScale(a.dom.insts, in), red, red[1], a.tol);
 		else residualDecision<1, false, false>(nullptr, s, normScale(a.dom.insts, in), red, red[1], a.tol);
 	});
@@ -765,10 +600,10 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 		// A: the update of the last direction (from the second pass on) and the finest restriction
 		nextPartials();
 		{
-			const PcgBlock *cblk = blocksOf(1);
+			const BlockTab *cblk = blocksOf(1);
 			const bool w4 = wide(0);
 			visit(0, a.mg.lv[1].tiles, a.mg.lv[1].ntiles * perA, perA, PHB_TILE_CELLS / perA, [&](int it, int b, int first) {
-				const PcgBlock &B = blk0[b];
+				const BlockTab &B = blk0[b];
 				const SysState &s = sst[B.inst];
 				if (s.done != RUNNING) return;
 				float *xb = s.saveBest ? a.xbest : nullptr;
@@ -787,7 +622,7 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 		if (!gridBarrier(a.ctrl)) return;
 		if (update) {
 			float *tmp = rIn; rIn = rOut; rOut = tmp;
-			running = pcgReduce<1>(ninst, pp, sst, itemRange, [&](SysState &s, int in, const double *red) {
+			running = reduceSystems<1, 1, -1>(ninst, pp, sst, itemRange, [&](SysState &s, int in, const double *red, double) {
 				const double crit = sqrt(red[0]) * normScale(a.dom.insts, in);
 				++s.it;
 				s.crit = crit;
@@ -807,7 +642,7 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 		}
 		update = true;
 		for (int l = 1; l < T; ++l) {
-			const PcgBlock *blk = blocksOf(l), *cblk = blocksOf(l + 1);
+			const BlockTab *blk = blocksOf(l), *cblk = blocksOf(l + 1);
 			const int per = perR(l);
 			const bool w4 = wide(l);
 			const PcgFine<false> f{a.mg.b[l], nullptr, a.mg.wd[l], 0.f};
@@ -820,14 +655,14 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 		pcgDense<D>(a.mg, sst);
 		if (!gridBarrier(a.ctrl)) return;
 		for (int l = T - 1; l >= 1; --l) {
-			const PcgBlock *blk = blocksOf(l), *cblk = blocksOf(l + 1);
+			const BlockTab *blk = blocksOf(l), *cblk = blocksOf(l + 1);
 			const float *bl = a.mg.b[l], *e = a.mg.x[l + 1];
 			float *xl = a.mg.x[l];
 			visit(2 * l + 1, a.mg.lv[l].tiles, a.mg.lv[l].ntiles * CPT, CPT, PHB_TILE, [&](int, int b, int first) {
-				const PcgBlock &B = blk[b];
+				const BlockTab &B = blk[b];
 				if (sst[B.inst].done != RUNNING) return;
 				const int c = first + int(threadIdx.x);
-				if (c >= B.ncells) return;
+				if (c >= B.cells()) return;
 				const int row = c / B.nx, z = D > 2 ? row / B.ny : 0;
 				const int g = B.off + c;
 				xl[g] = pcgProlongCell<D>(B, cblk[b], g, c - row * B.nx, row - z * B.ny, z, a.mg.lv[l].ncells, a.mg.A[l], a.mg.wd[l], bl[g], xl[g], e);
@@ -837,11 +672,11 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 		// finest level: z over t in place, (r, z)
 		nextPartials();
 		{
-			const PcgBlock *cblk = blocksOf(1);
+			const BlockTab *cblk = blocksOf(1);
 			const float *e = a.mg.x[1];
 			float *zz = a.mg.x[0];
 			visit(1, a.dom.tiles, n0, per0, cells0, [&](int it, int b, int l0) {
-				const PcgBlock &B = blk0[b];
+				const BlockTab &B = blk0[b];
 				if (sst[B.inst].done != RUNNING) return;
 				double acc[1] = {0};
 				if (al0) {
@@ -874,11 +709,11 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 			});
 		}
 		if (!gridBarrier(a.ctrl)) return;
-		pcgReduce<1>(ninst, pp, sst, tileRange, [&](SysState &s, int, const double *red) { pcgRho(s, red[0]); });
+		reduceSystems<1, 1, -1>(ninst, pp, sst, tileRange, [&](SysState &s, int, const double *red, double) { pcgRho(s, red[0]); });
 		// D: p' = z + beta p, q = A p', (p', q)
 		nextPartials();
 		visit(1, a.dom.tiles, n0, per0, cells0, [&](int it, int b, int l0) {
-			const PcgBlock &B = blk0[b];
+			const BlockTab &B = blk0[b];
 			const SysState &s = sst[B.inst];
 			if (s.done != RUNNING) return;
 			// a restart (p not yet written) takes p' = z: z + 0 * z
@@ -910,7 +745,7 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 			blockSumTo<1>(acc, pp + it);
 		});
 		if (!gridBarrier(a.ctrl)) return;
-		running = pcgReduce<1>(ninst, pp, sst, tileRange, [&](SysState &s, int, const double *red) {
+		running = reduceSystems<1, 1, -1>(ninst, pp, sst, tileRange, [&](SysState &s, int, const double *red, double) {
 			const double alpha = s.rho / red[0];
 			s.restart = 0;
 			if (!fin(alpha)) { s.done = NONFINITE; s.usedIt = s.it; }
@@ -921,10 +756,10 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 	// systems that stopped without converging return their best iterate (kRestoreBest)
 	if (a.xbest) {
 		visit(1, a.dom.tiles, n0, per0, cells0, [&](int, int b, int l0) {
-			const PcgBlock &B = blk0[b];
+			const BlockTab &B = blk0[b];
 			const SysState &s = sst[B.inst];
 			if (!((s.done == MAXIT || s.done == RISING) && s.bestIt >= 0 && s.best < s.crit)) return;
-			const int end = min(B.ncells, l0 + cells0);
+			const int end = min(B.cells(), l0 + cells0);
 			for (int l = l0 + int(threadIdx.x); l < end; l += PHB_TILE) a.x[B.off + l] = a.xbest[B.off + l];
 		});
 	}
@@ -970,13 +805,13 @@ int launchPcg(const phb_domain *dom, const phb_solve *sv, cudaStream_t s, bool s
 	const int rc = launchInit(a.st, dom->ninst, sv->tol, fromInner, a.maxit, a.ctrl, s);
 	if (rc) return rc;
 	const size_t stBytes = (size_t)dom->ninst * sizeof(SysState);
-	const size_t recBytes = (size_t)a.mg.nlevels * dom->nblocks * sizeof(PcgBlock);
+	const size_t recBytes = (size_t)a.mg.nlevels * dom->nblocks * sizeof(BlockTab);
 	if (stBytes > 160 * 1024) return setError(PHB_ERR_RANGE, "persistent solve: too many systems for the per-CTA state copy");
 	size_t smem = stBytes + recBytes;
-	if (recBytes > PCG_REC_MAX || smem > 160 * 1024) {
+	if (recBytes > TAB_SMEM_MAX || smem > 160 * 1024) {
 		smem = stBytes;
-		a.blocks = (PcgBlock *)(w + L.off[9]);
-		kPcgBlocks<D><<<std::max(1, std::min(1024, (dom->nblocks * a.mg.nlevels + 127) / 128)), 128, 0, s>>>(a.mg, (PcgBlock *)(w + L.off[9]));
+		a.blocks = (BlockTab *)(w + L.off[9]);
+		kPcgTabs<D><<<std::max(1, std::min(1024, (dom->nblocks * a.mg.nlevels + 127) / 128)), 128, 0, s>>>(a.mg, (BlockTab *)(w + L.off[9]));
 		PHB_CUDA(cudaGetLastError());
 	}
 	a.quarter = dom->ntiles < PCG_QUARTER_TILES;

@@ -485,84 +485,182 @@ __device__ __forceinline__ void blockSumTo(double (&v)[NV], double *dst) {
 	__syncthreads();
 }
 
-// Visit this CTA's tiles with the block record staged in sB.
-template <int D, typename F>
-__device__ __forceinline__ void forMyTiles(const Dom<double, D> &dom, int32_t *sB, F f) {
-	int staged = -1; // the block whose record sB holds (uniform over the CTA)
-	for (int tile = blockIdx.x; tile < dom.ntiles; tile += gridDim.x) {
-		const int b = __ldg(dom.tiles + 2 * tile);
-		const int l0 = __ldg(dom.tiles + 2 * tile + 1);
-		if (b != staged) {
-			__syncthreads();
-			if (threadIdx.x < PHB_BREC) sB[threadIdx.x] = __ldg(dom.blocks + b * PHB_BREC + threadIdx.x);
-			__syncthreads();
-			staged = b;
+// block tables -----------------------------------------------------------------------------
+// What the phases of a persistent kernel need of one block of one level, kept in shared memory for
+// the whole solve. The cell across a face that is not fixed is an affine function of the position
+// (periodic: the other end of the row; connected: phiPICT's axis mapping):
+// map[f] = c0 + cx x + cy y + cz z.
+struct __align__(16) BlockTab {
+	int nx, ny, nz, off;
+	int inst, instOff, instN;
+	unsigned int bits; // bit f: face f is not fixed; bit 8: rows of four may be loaded as vectors here and across every open face
+	int4 map[6];
+	__device__ __forceinline__ int cells() const { return nx * ny * nz; }
+	__device__ __forceinline__ bool open(int f) const { return (bits >> f) & 1; }
+	__device__ __forceinline__ bool rows4() const { return (bits >> 8) & 1; }
+};
+static_assert(sizeof(BlockTab) == 128, "BlockTab layout");
+constexpr size_t TAB_SMEM_MAX = 48 * 1024; // tables kept in shared memory up to this size, else in global memory
+
+template <int D>
+__device__ __forceinline__ void buildBlockTab(const int32_t *blocks, int b, BlockTab &o) {
+	const int32_t *B = blocks + b * PHB_BREC;
+	const int n[3] = {B[B_NX], B[B_NY], D > 2 ? B[B_NZ] : 1};
+	o.nx = n[0]; o.ny = n[1]; o.nz = n[2];
+	o.off = B[B_CELLOFF];
+	o.inst = B[B_INST];
+	o.instOff = B[B_INSTOFF];
+	o.instN = B[B_INSTN];
+	unsigned int open = 0;
+	bool al = ((n[0] | o.off) & 3) == 0;
+	for (int f = 0; f < 6; ++f) {
+		int4 m = make_int4(0, 0, 0, 0);
+		if (f < 2 * D && fType(B, f) != FT_FIXED) {
+			open |= 1u << f;
+			Dom<float, D> d;
+			d.blocks = blocks;
+			// the map from its values at the corner (0, 0, 0) of the face and one step along each
+			// tangential axis (the position along the face's own axis does not matter)
+			int v[4];
+			for (int k = 0; k < 4; ++k) {
+				Cell c;
+				c.B = B;
+				c.p[0] = c.p[1] = c.p[2] = 0;
+				c.p[f >> 1] = (f & 1) ? n[f >> 1] - 1 : 0;
+				if (k && k - 1 != (f >> 1) && n[k - 1] > 1) c.p[k - 1] = 1;
+				c.g = 0; c.mi = 0;
+				v[k] = (int)neighbor<float, D>(d, c, f).g;
+			}
+			m = make_int4(v[0], v[1] - v[0], v[2] - v[0], v[3] - v[0]);
+			if (f >= 2) al = al && m.y == 1 && ((m.x | m.z | m.w) & 3) == 0;
 		}
-		const int nc = sB[B_NX] * sB[B_NY] * (D > 2 ? sB[B_NZ] : 1);
-		f(tile, l0, nc);
+		o.map[f] = m;
 	}
+	o.bits = open | (al ? 256u : 0u);
+}
+__device__ __forceinline__ int tabMap(const int4 &m, int x, int y, int z) { return m.x + m.y * x + m.z * y + m.w * z; }
+
+// Indices of the neighbours of cell g (x, y, z), or of four cells of an aligned row from g on
+// (W = 4: the +x neighbour is that of the last one, the y and z neighbours start rows of four).
+// A face without neighbour gets g itself and no bit in `has`: every load is issued without a
+// branch, and what it brings is left out of the sum.
+template <int D, int W>
+__device__ __forceinline__ unsigned int tabNeighbors(const BlockTab &B, int g, int x, int y, int z, int (&o)[2 * D]) {
+	unsigned int has = (1u << (2 * D)) - 1;
+	const int sy = B.nx, sz = B.nx * B.ny;
+	o[0] = g - 1; o[1] = g + W; o[2] = g - sy; o[3] = g + sy;
+	if constexpr (D > 2) { o[4] = g - sz; o[5] = g + sz; }
+	bool end[2 * D];
+	end[0] = x == 0; end[1] = x + W == B.nx; end[2] = y == 0; end[3] = y + 1 == B.ny;
+	if constexpr (D > 2) { end[4] = z == 0; end[5] = z + 1 == B.nz; }
+#pragma unroll
+	for (int f = 0; f < 2 * D; ++f)
+		if (end[f]) {
+			if (B.open(f)) {
+				o[f] = tabMap(B.map[f], x, y, z);
+			} else {
+				o[f] = g;
+				has &= ~(1u << f);
+			}
+		}
+	return has;
 }
 
-// All CTAs: reduce every running system's partials (the group scheme of finalizeSystems) and
-// update the CTA's state copy; returns the number of systems still running.
-template <int K, int NQ, int INSTQ = -1, typename Fn>
-__device__ __forceinline__ int reduceStates(const int32_t *insts, int ninst, const double *partial, SysState *sst, Fn fn) {
-	constexpr int NV = NQ + 1;
+// Every CTA reduces the partials of every running system (K right-hand sides per instance, NQ
+// values each, [item][K][NQ]; items range(inst) = first, count) and updates its own copy of the
+// states: all the warps on few systems, a warp per system (four in flight) on many, each in the
+// order of finalizeSystems. With INSTQ >= 0 the last argument of fn is quantity INSTQ summed over
+// the instance's right-hand sides. Returns the systems still running.
+template <int K, int NQ, int INSTQ, typename Range, typename Fn>
+__device__ __forceinline__ int reduceSystems(int ninst, const double *pp, SysState *sst, Range range, Fn fn) {
+	constexpr int NV = NQ + (INSTQ >= 0 ? 1 : 0);
 	__shared__ int running;
 	__shared__ double gsm[NWARPS][NV];
-	if (threadIdx.x == 0) running = 0;
-	__syncthreads();
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const int nsys = ninst * K;
+	if (threadIdx.x == 0) running = 0;
+	auto load = [&](int item, int k, double (&a)[NV]) {
+		const double *p = pp + (size_t)item * K * NQ;
+#pragma unroll
+		for (int q = 0; q < NQ; ++q) a[q] += __ldcg(p + k * NQ + q);
+		if constexpr (INSTQ >= 0) {
+#pragma unroll
+			for (int kk = 0; kk < K; ++kk) a[NQ] += __ldcg(p + kk * NQ + INSTQ);
+		}
+	};
+	if (nsys >= NWARPS) {
+		constexpr int U = K == 1 ? 4 : 2;
+		__syncthreads();
+		int mine = 0;
+		for (int s0 = warp; s0 < nsys; s0 += U * NWARPS) {
+			double a0[U][NV];
+			bool act[U];
+#pragma unroll
+			for (int u = 0; u < U; ++u) {
+				const int s = s0 + u * NWARPS;
+				act[u] = s < nsys && sst[s].done == RUNNING;
+				double a1[NV];
+#pragma unroll
+				for (int q = 0; q < NV; ++q) a0[u][q] = a1[q] = 0;
+				if (act[u]) {
+					const int2 rg = range(s / K);
+					int t = lane;
+					for (; t + 32 < rg.y; t += 64) { load(rg.x + t, s % K, a0[u]); load(rg.x + t + 32, s % K, a1); }
+					if (t < rg.y) load(rg.x + t, s % K, a0[u]);
+				}
+#pragma unroll
+				for (int q = 0; q < NV; ++q) a0[u][q] += a1[q];
+			}
+#pragma unroll
+			for (int u = 0; u < U; ++u) {
+#pragma unroll
+				for (int q = 0; q < NV; ++q) a0[u][q] = warpSum(a0[u][q]);
+				if (act[u] && lane == u) fn(sst[s0 + u * NWARPS], (s0 + u * NWARPS) / K, a0[u], a0[u][NV - 1]);
+			}
+			if (lane < U) {
+				const int s = s0 + lane * NWARPS;
+				if (s < nsys && sst[s].done == RUNNING) ++mine;
+			}
+		}
+		if (mine) atomicAdd(&running, mine);
+		__syncthreads();
+		return running;
+	}
 	int G = NWARPS;
 	while (G > 1 && G * nsys > NWARPS) G >>= 1;
-	const int NG = NWARPS / G;
-	const int group = warp / G, wg = warp - group * G;
-	for (int base = 0; base < nsys; base += NG) {
-		const int s = base + group;
-		const bool act = s < nsys && sst[s].done == RUNNING;
-		double a0[NV], a1[NV];
+	const int s = warp / G, wg = warp - s * G;
+	const bool act = s < nsys && sst[s].done == RUNNING;
+	double a0[NV], a1[NV];
 #pragma unroll
-		for (int q = 0; q < NV; ++q) { a0[q] = 0; a1[q] = 0; }
+	for (int q = 0; q < NV; ++q) a0[q] = a1[q] = 0;
+	if (act) {
+		const int2 rg = range(s / K);
+		const int stride = G * 32;
+		int t = wg * 32 + lane;
+		for (; t + stride < rg.y; t += 2 * stride) { load(rg.x + t, s % K, a0); load(rg.x + t + stride, s % K, a1); }
+		if (t < rg.y) load(rg.x + t, s % K, a0);
+	}
+#pragma unroll
+	for (int q = 0; q < NV; ++q) {
+		const double v = warpSum(a0[q] + a1[q]);
+		if (lane == 0) gsm[warp][q] = v;
+	}
+	__syncthreads();
+	if (s < nsys && wg == 0 && lane == 0) {
 		if (act) {
-			const int inst = s / K, k = s - inst * K;
-			const int t0 = insts[inst * PHB_IREC + I_TILESTART], tc = insts[inst * PHB_IREC + I_TILECOUNT];
-			const int stride = G * 32;
-			auto load = [&](int t, double *a) {
-				const double *pp = partial + (size_t)(t0 + t) * K * NQ;
-#pragma unroll
-				for (int q = 0; q < NQ; ++q) a[q] += __ldcg(pp + k * NQ + q);
-				if (INSTQ >= 0) {
-#pragma unroll
-					for (int kk = 0; kk < K; ++kk) a[NQ] += __ldcg(pp + kk * NQ + (INSTQ < 0 ? 0 : INSTQ));
-				}
-			};
-			int t = wg * 32 + lane;
-			for (; t + stride < tc; t += 2 * stride) { load(t, a0); load(t + stride, a1); }
-			if (t < tc) load(t, a0);
-		}
-#pragma unroll
-		for (int q = 0; q < NV; ++q) {
-			const double v = warpSum(a0[q] + a1[q]);
-			if (lane == 0) gsm[warp][q] = v;
-		}
-		__syncthreads();
-		if (act && wg == 0 && lane == 0) {
 			double red[NV];
 #pragma unroll
 			for (int q = 0; q < NV; ++q) {
 				double v = 0;
-				for (int w = 0; w < G; ++w) v += gsm[group * G + w][q];
+				for (int w = 0; w < G; ++w) v += gsm[warp + w][q];
 				red[q] = v;
 			}
-			fn(sst[s], s / K, red, red[NQ]);
+			fn(sst[s], s / K, red, red[NV - 1]);
 		}
-		if (wg == 0 && lane == 0 && s < nsys && sst[s].done == RUNNING) atomicAdd(&running, 1);
-		__syncthreads();
+		if (sst[s].done == RUNNING) atomicAdd(&running, 1);
 	}
-	const int r = running;
 	__syncthreads();
-	return r;
+	return running;
 }
 
 // The reference stop rule of the first residual (kResidual) applied to a CTA state copy.
@@ -610,8 +708,8 @@ inline Layout solveLayout(const phb_domain *dom, int kind, int vecBytes, int nrh
 	const bool pcg = !plain && kind == 0 && vecBytes == 4 && nrhs == 1;
 	const size_t vb = align256((size_t)dom->ncells * nrhs * vecBytes);
 	for (int i = 0; i < vecCount(kind, pcg); ++i) { L.off[i] = o; o += vb; }
-	L.off[9] = o; // block tables of all levels (PcgBlock, pcg.cu)
-	if (pcg) o += align256((size_t)dom->nblocks * PHB_AMG_MAX_LEVELS * 128);
+	L.off[9] = o; // block tables (BlockTab), of every multigrid level for a preconditioned solve
+	if (!plain) o += align256((size_t)dom->nblocks * (pcg ? PHB_AMG_MAX_LEVELS : 1) * sizeof(BlockTab));
 	L.off[10] = o; // partials: two halves of up to 3 values per tile and right-hand side
 	o += align256((size_t)dom->ntiles * (pcg ? PCG_PARTIALS : nrhs * 3) * 2 * sizeof(double));
 	L.total = o;
@@ -640,6 +738,20 @@ inline int numSMs() {
 		cache[dev] = v;
 	}
 	return cache[dev];
+}
+
+// Initial state of system s: its tolerance from the options, or (fromInner) the one that the
+// refinement residual left in SysState::innerTol.
+__device__ __forceinline__ SysState initialState(const phb_tolerance &tol, int s, double innerTol, int fromInner, int maxit) {
+	SysState z;
+	memset(&z, 0, sizeof(z));
+	z.tol = fromInner ? innerTol : tol.mode == 0 ? tol.atol : tol.mode == 2 ? tol.values[s] : NAN; // NAN: resolved from the right-hand side
+	z.innerTol = z.tol;
+	z.maxit = maxit;
+	z.best = INFINITY;
+	z.restart = 1;
+	z.bestIt = -1;
+	return z;
 }
 
 // kInit launched on `s`: the initial state of the nsys systems of a solve (krylov.cu)

@@ -1,0 +1,107 @@
+"""The persistent CG and BiCGStab (grid-wide and one cluster per instance) against the per-phase
+kernels: the same bits, on the shapes where the work split can go wrong: rows of four, odd rows,
+partial tiles, one cell thick blocks, rotated connections, instances of 1 to 33 tiles (a cluster
+holds at most 32), batches of few and many systems, best iterates of solves cut off early."""
+import pytest
+import torch
+
+import phipict_b200 as pb
+from phipict_b200 import _C
+from phipict_b200.solvers import BICGSTAB, CG, solver_for
+from cases import duct_3d, hartmann_2d, rotated_pair_2d, seeded_state
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    "row4_3d": lambda **k: duct_3d(16, 12, 8, 2, **k),
+    "odd_3d": lambda **k: duct_3d(13, 11, 9, 3, **k),
+    "thin_3d": lambda **k: duct_3d(20, 1, 24, 1, **k),
+    "wide_3d": lambda **k: duct_3d(48, 40, 20, 2, **k),        # 76 tiles: the grid kernel
+    "wide_odd_3d": lambda **k: duct_3d(37, 25, 23, 2, **k),
+    "rotated_2d": lambda **k: rotated_pair_2d(16, **k),
+    "one_tile": lambda **k: hartmann_2d(32, 24, **k),
+    "two_tiles": lambda **k: hartmann_2d(64, 32, **k),
+    "three_tiles_odd": lambda **k: hartmann_2d(51, 53, **k),
+    "sixteen_tiles_odd": lambda **k: hartmann_2d(129, 121, **k),
+    "seventeen_tiles": lambda **k: hartmann_2d(128, 129, **k),  # two tiles per CTA from here
+    "thirty_two_tiles": lambda **k: hartmann_2d(181, 181, **k),
+    "thirty_three_tiles": lambda **k: hartmann_2d(184, 180, **k),
+    "batch_of_copies": lambda **k: hartmann_2d(33, 31, batch=3, **k),
+}
+
+
+def _assemble(dom, seed):
+    ts = torch.tensor([0.01], dtype=torch.float64)
+    _C.SetupAdvectionMatrix(dom, ts, 0)
+    _C.SetupPressureMatrix(dom, ts)
+
+
+def _rhs(dom, n, nrhs, seed):
+    g = torch.Generator().manual_seed(seed)
+    b = torch.randn(n * nrhs, generator=g, dtype=torch.float64).to(dom.getDtype()).to(dom.getDevice())
+    dom._subtract_mean(b, nrhs)
+    return b
+
+
+def _solve(dom, kind, nrhs, A, b, tol, maxit, mode, best=False, ctas=0):
+    s = solver_for(dom, kind, dom.getDtype(), nrhs, tag=f"m{mode}c{ctas}")
+    x = torch.zeros_like(b)
+    s.solve(A, b, x, tol, maxit, return_best=best, use_graph=mode, ctas_per_sm=ctas)
+    return x, s.results()
+
+
+def _same(a, b):
+    return torch.equal(a[0], b[0]) and [(i.usedIterations, i.finalResidual, i.status) for i in a[1]] == [
+        (i.usedIterations, i.finalResidual, i.status) for i in b[1]]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64], ids=["f32", "f64"])
+@pytest.mark.parametrize("case", list(CASES))
+def test_persistent_solvers_match_per_phase_kernels(cuda, case, dtype):
+    dom = CASES[case](dtype=dtype)
+    seeded_state(dom, 5, scale=0.2)
+    dom.PrepareSolve()
+    _assemble(dom, 5)
+    n = dom.numCells()
+    d = dom.getSpatialDims()
+    tol = 1e-4
+    b = _rhs(dom, n, 1, 7)
+    ref = _solve(dom, CG, 1, dom._P_st, b, tol, 3000, 1)
+    assert all(i.converged for i in ref[1])
+    assert _same(_solve(dom, CG, 1, dom._P_st, b, tol, 3000, 2), ref)          # a cluster per instance up to 32 tiles
+    assert _same(_solve(dom, CG, 1, dom._P_st, b, tol, 3000, 2, ctas=1), ref)  # the grid kernel
+    # cut off before convergence: the best iterate
+    ref = _solve(dom, CG, 1, dom._P_st, b, 1e-30, 7, 1, best=True)
+    for ctas in (0, 1):
+        assert _same(_solve(dom, CG, 1, dom._P_st, b, 1e-30, 7, 2, best=True, ctas=ctas), ref)
+    for nrhs in (1, d):
+        b = _rhs(dom, n, nrhs, 9)
+        ref = _solve(dom, BICGSTAB, nrhs, dom._C_st, b, 1e-5, 500, 1)
+        assert all(i.converged for i in ref[1])
+        assert _same(_solve(dom, BICGSTAB, nrhs, dom._C_st, b, 1e-5, 500, 2), ref)
+        if nrhs > 1:
+            ref = _solve(dom, CG, nrhs, dom._P_st, b, tol, 3000, 1)
+            assert _same(_solve(dom, CG, nrhs, dom._P_st, b, tol, 3000, 2), ref)
+
+
+@pytest.mark.parametrize("sizes", [((16, 12), (33, 20), (64, 48)),
+                                   ((16, 12), (13, 9), (64, 48), (33, 20), (8, 8), (6, 10), (40, 36), (21, 7), (12, 12), (96, 50), (5, 4))],
+                         ids=["few", "many"])
+def test_persistent_solvers_of_a_batch(cuda, sizes):
+    """Instances that stop after different counts, in one launch: the per-phase kernels' bits."""
+    doms = []
+    for k, (nx, ny) in enumerate(sizes):
+        m = hartmann_2d(nx, ny)
+        seeded_state(m, 60 + k, scale=0.2)
+        m.PrepareSolve()
+        doms.append(m)
+    batch = pb.DomainBatch(doms)
+    _assemble(batch, 3)
+    b = _rhs(batch, batch.numCells(), 1, 3)
+    ref = _solve(batch, CG, 1, batch._P_st, b, 1e-6, 3000, 1)
+    assert len({i.usedIterations for i in ref[1]}) > 1
+    for ctas in (0, 1):
+        assert _same(_solve(batch, CG, 1, batch._P_st, b, 1e-6, 3000, 2, ctas=ctas), ref)
+    b = _rhs(batch, batch.numCells(), 2, 4)
+    ref = _solve(batch, BICGSTAB, 2, batch._C_st, b, 1e-8, 500, 1)
+    assert _same(_solve(batch, BICGSTAB, 2, batch._C_st, b, 1e-8, 500, 2), ref)
