@@ -1,5 +1,6 @@
 // The persistent Krylov solvers: one cooperative launch runs a whole CG or BiCGStab solve, with
-// grid barriers between its phases (phb_krylov.cuh). The multigrid-preconditioned CG is in pcg.cu.
+// grid barriers between its phases (phb_krylov.cuh). The multigrid-preconditioned CG is in pcg.cu,
+// the CG of small instances in cluster_cg.cu.
 //
 // What bounds a phase on grids that fit L2: the barrier (1.2 to 1.6 us) and the chain of dependent
 // L2 round trips after it; on larger grids, bytes in flight. Block tables and the CTA's tile list
@@ -570,6 +571,13 @@ template <typename T, int D, int K>
 int launchPersistent(const phb_domain *dom, const phb_solve *sv, cudaStream_t s, bool stopStart, int fromInner) {
 	if constexpr (std::is_same<T, float>::value && K == 1) {
 		if (sv->amg && sv->kind == 0) return launchPcg<D>(dom, sv, s, stopStart, fromInner);
+	}
+	if constexpr (K == 1) {
+		if (sv->kind == 0) {
+			bool taken = false;
+			const int rc = launchClusterCg<T, D>(dom, sv, s, stopStart, fromInner, &taken);
+			if (rc || taken) return rc;
+		}
 	}
 	Dom<double, D> dm(*dom);
 	const Layout L = solveLayout(dom, sv->kind, sizeof(T), K);

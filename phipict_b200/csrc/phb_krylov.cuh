@@ -757,6 +757,10 @@ __device__ __forceinline__ SysState initialState(const phb_tolerance &tol, int s
 // kInit launched on `s`: the initial state of the nsys systems of a solve (krylov.cu)
 int launchInit(SysState *st, int nsys, const phb_tolerance &tol, int fromInner, int maxit, Control *ctrl, cudaStream_t s);
 
+// The CG of small instances as one cluster per instance (cluster_cg.cu); *taken: whether it applies.
+template <typename T, int D>
+int launchClusterCg(const phb_domain *dom, const phb_solve *sv, cudaStream_t s, bool stopStart, int fromInner, bool *taken);
+
 // A persistent preconditioned CG recorded on `s` (pcg.cu).
 template <int D>
 int launchPcg(const phb_domain *dom, const phb_solve *sv, cudaStream_t s, bool stopStart, int fromInner);
