@@ -483,7 +483,7 @@ __global__ void kRefineUpdate(int64_t n, double *__restrict__ x, const float *__
 	for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) x[i] += double(e[i]);
 }
 
-__global__ void kInitOuter(SysState *st, int nsys, phb_tolerance tol, Control *ctrl, int maxLoops, LoopCond arm) {
+__global__ void kInitOuter(SysState *st, int nsys, phb_tolerance tol, Control *ctrl, int maxLoops) {
 	for (int s = threadIdx.x; s < nsys; s += blockDim.x) {
 		SysState z;
 		memset(&z, 0, sizeof(z));
@@ -492,7 +492,6 @@ __global__ void kInitOuter(SysState *st, int nsys, phb_tolerance tol, Control *c
 	}
 	if (threadIdx.x == 0) {
 		ctrl->counter = 0; ctrl->allDone = 0; ctrl->loops = 0; ctrl->maxLoops = maxLoops;
-		if (arm.active) cudaGraphSetConditional(arm.handle, 1u);
 	}
 }
 
@@ -1062,29 +1061,36 @@ static int emitRefine(const phb_domain *dom, const phb_refine *rf, cudaStream_t 
 		const int rc0 = createCondition(s, &outerHandle);
 		if (rc0) return rc0;
 	}
-	kInitOuter<<<1, 256, 0, s>>>(stO, nsys, rf->tol, ctrlO, rf->max_outer + 2, LoopCond{outerHandle, graph ? 1 : 0});
+	kInitOuter<<<1, 256, 0, s>>>(stO, nsys, rf->tol, ctrlO, rf->max_outer + 2);
 	PHB_CUDA(cudaGetLastError());
-	auto outer = [&](cudaStream_t os, LoopCond lc) -> int {
+	// The residual comes before the loop and at the end of its body, so that a system that needs no
+	// (further) correction starts no inner solve: the pass of the loop that would only have found
+	// that out cost 20 to 40 us a solve.
+	auto residual = [&](cudaStream_t os, LoopCond lc) -> int {
 		kRefineResidual<D, K><<<dom->ntiles, PHB_TILE, 0, os>>>(dm, rf->A64, rf->b, rf->x, r32, e32, stO, partial, ctrlO,
 			rf->inner_rtol, rf->max_outer, rf->tol, stI, lc);
-		int rc = checkLaunch("kRefineResidual");
-		if (rc) return rc;
-		rc = emitSolve<float, D, K>(dom, &in, os, ss, graph ? 2 : 0, true, 1);
+		return checkLaunch("kRefineResidual");
+	};
+	auto sweep = [&](cudaStream_t os, LoopCond lc) -> int {
+		int rc = emitSolve<float, D, K>(dom, &in, os, ss, graph ? 2 : 0, true, 1);
 		if (rc) return rc;
 		kRefineUpdate<K><<<gridFor(dom->ncells * K), 256, 0, os>>>(dom->ncells * K, rf->x, e32);
-		return checkLaunch("kRefineUpdate");
+		rc = checkLaunch("kRefineUpdate");
+		if (rc) return rc;
+		return residual(os, lc);
 	};
-	if (graph) return addWhile(s, ss.s[1], outerHandle, outer);
+	int rc = residual(s, LoopCond{outerHandle, graph ? 1 : 0});
+	if (rc) return rc;
+	if (graph) return addWhile(s, ss.s[1], outerHandle, sweep);
 	// host loop: every kernel launched on its own (profilers see each launch)
 	int *hflag = nullptr;
 	PHB_CUDA(cudaMallocHost(&hflag, sizeof(int)));
-	int rc = PHB_OK;
-	for (int sweep = 0; sweep < rf->max_outer + 2; ++sweep) {
-		rc = outer(s, LoopCond{0, 0});
-		if (rc) break;
+	for (int k = 0; k < rf->max_outer + 2; ++k) {
 		cudaMemcpyAsync(hflag, &ctrlO->allDone, sizeof(int), cudaMemcpyDeviceToHost, s);
 		cudaStreamSynchronize(s);
 		if (*hflag) break;
+		rc = sweep(s, LoopCond{0, 0});
+		if (rc) break;
 	}
 	cudaFreeHost(hflag);
 	return rc;
