@@ -19,11 +19,11 @@
 // are formed before its loads, and the loads are issued without a branch between them: a face
 // resolved by a branch of its own costs its own round trip to L2, which made most of an iteration
 // of the form before this one. Microseconds per iteration, before and after (B200):
-//   3 blocks 64x48x48 (442,368 cells, rows of four)          67 -> 45
-//   2 blocks 37x45x41 (136,530 cells, odd rows)               72 -> 42
-//   128^3 (2.1 M cells)                                      213 -> 108
-//   64 2D instances of 32^2 to 256^2 (1.2 M cells)           170 -> 92
-//   6 3D instances of 32^3 to 112^3 (3.6 M cells, odd rows)  430 -> 255
+//   3 blocks 64x48x48 (442,368 cells, rows of four)          67 -> 44
+//   2 blocks 37x45x41 (136,530 cells, odd rows)               72 -> 41
+//   128^3 (2.1 M cells)                                      213 -> 104
+//   64 2D instances of 32^2 to 256^2 (1.2 M cells)           170 -> 91
+//   6 3D instances of 32^3 to 112^3 (3.6 M cells, odd rows)  430 -> 247
 #include "phb_krylov.cuh"
 
 namespace phb {
@@ -455,11 +455,15 @@ __device__ __forceinline__ void pcgDense(const AmgView<D> &mg, const SysState *s
 	}
 }
 
+template <int N>
+using Count = std::integral_constant<int, N>;
+
 template <int D>
 __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgArgs<D> a) {
 	extern __shared__ __align__(16) SysState sst[];
 	__shared__ int2 sItem[(2 * AMG_MAX_LEVELS) * PCG_ITEMS]; // slot 2l: restriction of level l, 2l+1: its prolongation
 	__shared__ unsigned int sAl;
+	__shared__ double ws[TILE_SUMS * 2 * NWARPS];
 	const int ninst = a.dom.ninst;
 	const int nblk = a.dom.nblocks;
 	const int T = a.mg.nlevels - 1;
@@ -501,6 +505,8 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 		sItem[i] = w;
 	}
 	__syncthreads();
+	int ph = 0;
+	double *pp = a.partial;
 	// visit this CTA's items of a slot: f(item, block, first cell)
 	auto visit = [&](int slot, const int32_t *tiles, int n, int per, int cells, auto f) {
 		int k = 0;
@@ -509,13 +515,25 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 			f(it, w.x, w.y);
 		}
 	};
+	// the same with sums over every item into the phase's partials: f(block, first cell, values)
+	auto visitSums = [&](auto count, int slot, const int32_t *tiles, int n, int per, int cells, auto f) {
+		constexpr int NV = decltype(count)::value;
+		TileSums<NV> sums{reinterpret_cast<double (*)[NV][NWARPS]>(ws), pp, 0};
+		visit(slot, tiles, n, per, cells, [&](int, int b, int first) {
+			double acc[NV];
+#pragma unroll
+			for (int q = 0; q < NV; ++q) acc[q] = 0;
+			f(b, first, acc);
+			sums.add(acc);
+			sums.next();
+		});
+		sums.finish();
+	};
 	const int64_t N = a.dom.ncells;
 	const BlockTab *blk0 = blocksOf(0);
 	const bool al0 = (alMask & 1) && !quarter;
 	const int perA = perR(0);
 	const int n0 = a.dom.ntiles * per0;
-	int ph = 0;
-	double *pp = a.partial;
 	auto nextPartials = [&] { pp = a.partial + (size_t)(ph++ & 1) * a.half; };
 	auto tileRange = [&](int inst) {
 		const int32_t *in = a.dom.insts + inst * PHB_IREC;
@@ -552,10 +570,9 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 	float *rIn = a.r0, *rOut = a.r1, *pIn = a.p0, *pOut = a.p1;
 	// r = b - A x, (r, r), (b, b)
 	nextPartials();
-	visit(1, a.dom.tiles, n0, per0, cells0, [&](int it, int b, int l0) {
+	visitSums(Count<2>{}, 1, a.dom.tiles, n0, per0, cells0, [&](int b, int l0, double (&acc)[2]) {
 		const BlockTab &B = blk0[b];
 		if (sst[B.inst].done != RUNNING) return;
-		double acc[2] = {0, 0};
 		const FX<float> fx{a.x};
 		if (al0) {
 			quad(B, l0, [&](int g, int x, int y, int z) {
@@ -587,7 +604,6 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 					}
 			});
 		}
-		blockSumTo<2>(acc, pp + (size_t)it * 2);
 	});
 	if (!gridBarrier(a.ctrl)) return;
 	int running = reduceSystems<1, 2, -1>(ninst, pp, sst, tileRange, [&](SysState &s, int in, const double *red, double) {
@@ -602,17 +618,15 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 		{
 			const BlockTab *cblk = blocksOf(1);
 			const bool w4 = wide(0);
-			visit(0, a.mg.lv[1].tiles, a.mg.lv[1].ntiles * perA, perA, PHB_TILE_CELLS / perA, [&](int it, int b, int first) {
+			visitSums(Count<1>{}, 0, a.mg.lv[1].tiles, a.mg.lv[1].ntiles * perA, perA, PHB_TILE_CELLS / perA, [&](int b, int first, double (&acc)[1]) {
 				const BlockTab &B = blk0[b];
 				const SysState &s = sst[B.inst];
 				if (s.done != RUNNING) return;
 				float *xb = s.saveBest ? a.xbest : nullptr;
 				if (update) {
 					const PcgFine<true> f{rIn, a.q, a.mg.wd[0], float(s.alpha)};
-					double acc[1];
 					if (w4) acc[0] = pcgRestrictItem<D, 4, true>(B, cblk[b], first, N, a.A, f, a.mg.x[0], a.mg.b[1], rOut, a.x, pIn, xb);
 					else acc[0] = pcgRestrictItem<D, 2, true>(B, cblk[b], first, N, a.A, f, a.mg.x[0], a.mg.b[1], rOut, a.x, pIn, xb);
-					blockSumTo<1>(acc, pp + it);
 				} else {
 					const PcgFine<false> f{rIn, nullptr, a.mg.wd[0], 0.f};
 					pcgRestrictItemAny<D>(w4, B, cblk[b], first, N, a.A, f, a.mg.x[0], a.mg.b[1]);
@@ -675,10 +689,9 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 			const BlockTab *cblk = blocksOf(1);
 			const float *e = a.mg.x[1];
 			float *zz = a.mg.x[0];
-			visit(1, a.dom.tiles, n0, per0, cells0, [&](int it, int b, int l0) {
+			visitSums(Count<1>{}, 1, a.dom.tiles, n0, per0, cells0, [&](int b, int l0, double (&acc)[1]) {
 				const BlockTab &B = blk0[b];
 				if (sst[B.inst].done != RUNNING) return;
-				double acc[1] = {0};
 				if (al0) {
 					quad(B, l0, [&](int g, int x, int y, int z) {
 						float rv[4], tv[4], out[4];
@@ -705,20 +718,18 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 							}
 					});
 				}
-				blockSumTo<1>(acc, pp + it);
 			});
 		}
 		if (!gridBarrier(a.ctrl)) return;
 		reduceSystems<1, 1, -1>(ninst, pp, sst, tileRange, [&](SysState &s, int, const double *red, double) { pcgRho(s, red[0]); });
 		// D: p' = z + beta p, q = A p', (p', q)
 		nextPartials();
-		visit(1, a.dom.tiles, n0, per0, cells0, [&](int it, int b, int l0) {
+		visitSums(Count<1>{}, 1, a.dom.tiles, n0, per0, cells0, [&](int b, int l0, double (&acc)[1]) {
 			const BlockTab &B = blk0[b];
 			const SysState &s = sst[B.inst];
 			if (s.done != RUNNING) return;
 			// a restart (p not yet written) takes p' = z: z + 0 * z
 			const FDir<float> fd{z0, s.restart ? z0 : pIn, s.restart ? 0.f : float(s.beta), false};
-			double acc[1] = {0};
 			if (al0) {
 				quad(B, l0, [&](int g, int x, int y, int z) {
 					float yv[4], fc[4];
@@ -742,7 +753,6 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 						}
 				});
 			}
-			blockSumTo<1>(acc, pp + it);
 		});
 		if (!gridBarrier(a.ctrl)) return;
 		running = reduceSystems<1, 1, -1>(ninst, pp, sst, tileRange, [&](SysState &s, int, const double *red, double) {
@@ -816,7 +826,7 @@ int launchPcg(const phb_domain *dom, const phb_solve *sv, cudaStream_t s, bool s
 	}
 	a.quarter = dom->ntiles < PCG_QUARTER_TILES;
 	auto kern = kPcg<D>;
-	if (smem > 40 * 1024) PHB_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+	if (smem > 32 * 1024) PHB_CUDA(allowSmem((const void *)kern));
 	int perSM = 0;
 	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, PHB_TILE, smem) != cudaSuccess || perSM < 1) perSM = 1;
 	if (sv->ctas_per_sm > 0) perSM = std::min(perSM, sv->ctas_per_sm);

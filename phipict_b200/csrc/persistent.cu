@@ -10,9 +10,9 @@
 // over a warp for every row length, and the inner products are formed through shared memory in
 // the order of four consecutive cells per thread: the same bits as the per-phase kernels.
 // Measured (B200, microseconds per iteration, before -> after): CG float64 on 442,368 cells 16.6 ->
-// 15.3 and on 3.3 M cells 99 -> 96; BiCGStab float32 with three right-hand sides inside a
-// refinement on 442,368 cells 77 -> 68, on 136,530 cells (odd rows) 86 -> 70, on 2.1 M 286 -> 243,
-// with two on 64 2D instances (1.2 M) 180 -> 130.
+// 15.4 and on 3.3 M cells 99 -> 91; BiCGStab float32 with three right-hand sides inside a
+// refinement on 442,368 cells 77 -> 65, on 136,530 cells (odd rows) 86 -> 69, on 2.1 M 286 -> 223,
+// with two on 64 2D instances (1.2 M) 180 -> 120.
 #include "phb_krylov.cuh"
 
 namespace phb {
@@ -28,14 +28,28 @@ struct TileCtx {
 	T *stage; // two tiles of values for the inner products of unaligned rows
 	bool vec; // operands on 16-byte boundaries
 
-	// f(tile, block, first cell) for every tile of this CTA
+	// f(block, first cell) for every tile of this CTA
 	template <typename F>
 	__device__ __forceinline__ void tiles(F f) const {
 		int k = 0;
 		for (int t = blockIdx.x; t < dom.ntiles; t += gridDim.x, ++k) {
 			const int2 w = k < TILE_ITEMS ? items[k] : make_int2(__ldg(dom.tiles + 2 * t), __ldg(dom.tiles + 2 * t + 1));
-			f(t, blk[w.x], w.y);
+			f(blk[w.x], w.y);
 		}
+	}
+	// the same with sums over every tile into dst: f(block, first cell, values)
+	template <int NV, typename F>
+	__device__ __forceinline__ void tileSums(double *dst, double *ws, F f) const {
+		TileSums<NV> sums{reinterpret_cast<double (*)[NV][NWARPS]>(ws), dst, 0};
+		tiles([&](const BlockTab &B, int l0) {
+			double acc[NV];
+#pragma unroll
+			for (int q = 0; q < NV; ++q) acc[q] = 0;
+			f(B, l0, acc);
+			sums.add(acc);
+			sums.next();
+		});
+		sums.finish();
 	}
 	__device__ __forceinline__ bool rows4(const BlockTab &B) const {
 		return vec && B.rows4() && (K == 1 || ((B.instOff | B.instN) & 3) == 0);
@@ -230,6 +244,7 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 	extern __shared__ __align__(16) SysState sst[];
 	__shared__ int2 items[TILE_ITEMS];
 	__shared__ __align__(16) T stage[2 * PHB_TILE_CELLS];
+	__shared__ double ws[TILE_SUMS * 2 * K * NWARPS];
 	const TileCtx<T, D, K> cx = tileContext<T, D, K>(dom, blocks, sst, st, items, stage);
 	const int64_t N = dom.ncells;
 	auto range = [&](int inst) {
@@ -243,16 +258,12 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 	double *pp = partial;
 	// r = b - A x, (r, r), (b, b)
 	pp = partial + (size_t)(ph++ & 1) * half;
-	cx.tiles([&](int tile, const BlockTab &B, int l0) {
+	cx.template tileSums<2 * K>(pp, ws, [&](const BlockTab &B, int l0, double (&acc)[2 * K]) {
 		bool act[K];
 		FX<T> fx[K];
 #pragma unroll
 		for (int k = 0; k < K; ++k) { act[k] = sst[B.inst * K + k].done == RUNNING; fx[k].x = x; }
-		double acc[2 * K];
-#pragma unroll
-		for (int k = 0; k < 2 * K; ++k) acc[k] = 0;
 		residualTile<T, D, K>(cx, B, l0, N, A, b, act, fx, acc, [&](int64_t o, int n, const T (&rv)[4]) { put(r + o, n, rv); });
-		blockSumTo<2 * K>(acc, pp + (size_t)tile * 2 * K);
 	});
 	if (!gridBarrier(ctrl)) return;
 	int running = reduceSystems<K, 2, 1>(dom.ninst, pp, sst, range, [&](SysState &s, int in, const double *red, double bb) {
@@ -262,7 +273,7 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 	for (int iter = 0; running > 0 && iter <= maxit + 1; ++iter) {
 		// p' = r + beta p, q = A p', (p', q)
 		pp = partial + (size_t)(ph++ & 1) * half;
-		cx.tiles([&](int tile, const BlockTab &B, int l0) {
+		cx.template tileSums<K>(pp, ws, [&](const BlockTab &B, int l0, double (&acc)[K]) {
 			bool act[K];
 			FDir<T> fd[K];
 #pragma unroll
@@ -272,16 +283,12 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 				// a restart (p not yet written) takes p' = r: r + 0 r
 				fd[k] = FDir<T>{r, s.restart ? r : pIn, s.restart ? T(0) : T(s.beta), false};
 			}
-			double acc[K];
-#pragma unroll
-			for (int k = 0; k < K; ++k) acc[k] = 0;
 			tilePhase<T, D, K>(cx, B, l0, N, A, act, fd, acc,
 				[&](int, int64_t o, int n, const T (&y)[4], const T (&f)[4]) { put(pOut + o, n, f); put(q + o, n, y); },
 				[&](int k, int64_t, int, const T (&y)[4], const T (&f)[4], double (&ac)[K]) {
 #pragma unroll
 					for (int i = 0; i < 4; ++i) ac[k] = fma(double(f[i]), double(y[i]), ac[k]);
 				});
-			blockSumTo<K>(acc, pp + (size_t)tile * K);
 		});
 		if (!gridBarrier(ctrl)) return;
 		reduceSystems<K, 1, -1>(dom.ninst, pp, sst, range, [&](SysState &s, int, const double *red, double) {
@@ -292,10 +299,7 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 		});
 		// x += alpha p', r -= alpha q, (r, r)
 		pp = partial + (size_t)(ph++ & 1) * half;
-		cx.tiles([&](int tile, const BlockTab &B, int l0) {
-			double acc[K];
-#pragma unroll
-			for (int k = 0; k < K; ++k) acc[k] = 0;
+		cx.template tileSums<K>(pp, ws, [&](const BlockTab &B, int l0, double (&acc)[K]) {
 			const int l = l0 + 4 * int(threadIdx.x);
 			const int n = max(0, min(4, B.cells() - l));
 			const bool al = cx.rows4(B) && n == 4;
@@ -320,7 +324,6 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 				st4(x + o, n, al, xv);
 				st4(r + o, n, al, rv);
 			}
-			blockSumTo<K>(acc, pp + (size_t)tile * K);
 		});
 		if (!gridBarrier(ctrl)) return;
 		running = reduceSystems<K, 1, -1>(dom.ninst, pp, sst, range, [&](SysState &s, int in, const double *red, double) {
@@ -348,7 +351,7 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 	}
 	// systems that stopped without converging return their best iterate (kRestoreBest)
 	if (xbest) {
-		cx.tiles([&](int, const BlockTab &B, int l0) {
+		cx.tiles([&](const BlockTab &B, int l0) {
 			const int end = min(B.cells(), l0 + PHB_TILE_CELLS);
 #pragma unroll
 			for (int k = 0; k < K; ++k) {
@@ -387,6 +390,7 @@ __global__ void __launch_bounds__(PHB_TILE, 2) kBicgPersistent(Dom<double, D> do
 	extern __shared__ __align__(16) SysState sst[];
 	__shared__ int2 items[TILE_ITEMS];
 	__shared__ __align__(16) T stage[2 * PHB_TILE_CELLS];
+	__shared__ double ws[TILE_SUMS * 3 * K * NWARPS];
 	const TileCtx<T, D, K> cx = tileContext<T, D, K>(dom, blocks, sst, st, items, stage);
 	const int64_t N = dom.ncells;
 	auto range = [&](int inst) {
@@ -399,19 +403,15 @@ __global__ void __launch_bounds__(PHB_TILE, 2) kBicgPersistent(Dom<double, D> do
 	int ph = 0;
 	double *pp = partial;
 	pp = partial + (size_t)(ph++ & 1) * half;
-	cx.tiles([&](int tile, const BlockTab &B, int l0) {
+	cx.template tileSums<2 * K>(pp, ws, [&](const BlockTab &B, int l0, double (&acc)[2 * K]) {
 		bool act[K];
 		FX<T> fx[K];
 #pragma unroll
 		for (int k = 0; k < K; ++k) { act[k] = sst[B.inst * K + k].done == RUNNING; fx[k].x = x; }
-		double acc[2 * K];
-#pragma unroll
-		for (int k = 0; k < 2 * K; ++k) acc[k] = 0;
 		residualTile<T, D, K>(cx, B, l0, N, A, b, act, fx, acc, [&](int64_t o, int n, const T (&rv)[4]) {
 			put(r + o, n, rv);
 			put(r0 + o, n, rv);
 		});
-		blockSumTo<2 * K>(acc, pp + (size_t)tile * 2 * K);
 	});
 	if (!gridBarrier(ctrl)) return;
 	int running = reduceSystems<K, 2, 1>(dom.ninst, pp, sst, range, [&](SysState &s, int in, const double *red, double bb) {
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(PHB_TILE, 2) kBicgPersistent(Dom<double, D> do
 	for (int iter = 0; running > 0 && iter <= maxit + 1; ++iter) {
 		// p = r + beta (p - omega v), v = A p, (r0, v)
 		pp = partial + (size_t)(ph++ & 1) * half;
-		cx.tiles([&](int tile, const BlockTab &B, int l0) {
+		cx.template tileSums<K>(pp, ws, [&](const BlockTab &B, int l0, double (&acc)[K]) {
 			bool act[K];
 			FBicgP<T> fp[K];
 #pragma unroll
@@ -432,9 +432,6 @@ __global__ void __launch_bounds__(PHB_TILE, 2) kBicgPersistent(Dom<double, D> do
 				const bool rs = s.restart;
 				fp[k] = FBicgP<T>{r, rs ? r : pIn, rs ? r : vIn, rs ? T(0) : T(s.beta), rs ? T(0) : T(s.omega), false};
 			}
-			double acc[K];
-#pragma unroll
-			for (int k = 0; k < K; ++k) acc[k] = 0;
 			tilePhase<T, D, K>(cx, B, l0, N, A, act, fp, acc,
 				[&](int, int64_t o, int n, const T (&y)[4], const T (&f)[4]) { put(pOut + o, n, f); put(vOut + o, n, y); },
 				[&](int k, int64_t o, int n, const T (&y)[4], const T (&)[4], double (&ac)[K]) {
@@ -443,7 +440,6 @@ __global__ void __launch_bounds__(PHB_TILE, 2) kBicgPersistent(Dom<double, D> do
 #pragma unroll
 					for (int i = 0; i < 4; ++i) ac[k] = fma(double(w[i]), double(y[i]), ac[k]);
 				});
-			blockSumTo<K>(acc, pp + (size_t)tile * K);
 		});
 		if (!gridBarrier(ctrl)) return;
 		reduceSystems<K, 1, -1>(dom.ninst, pp, sst, range, [&](SysState &s, int, const double *red, double) {
@@ -454,7 +450,7 @@ __global__ void __launch_bounds__(PHB_TILE, 2) kBicgPersistent(Dom<double, D> do
 		});
 		// s = r - alpha v, t = A s, (t,s), (t,t), (s,s)
 		pp = partial + (size_t)(ph++ & 1) * half;
-		cx.tiles([&](int tile, const BlockTab &B, int l0) {
+		cx.template tileSums<3 * K>(pp, ws, [&](const BlockTab &B, int l0, double (&acc)[3 * K]) {
 			bool act[K];
 			FBicgS<T> fs[K];
 #pragma unroll
@@ -463,9 +459,6 @@ __global__ void __launch_bounds__(PHB_TILE, 2) kBicgPersistent(Dom<double, D> do
 				act[k] = s.done == RUNNING;
 				fs[k] = FBicgS<T>{r, vOut, T(s.alpha)};
 			}
-			double acc[3 * K];
-#pragma unroll
-			for (int k = 0; k < 3 * K; ++k) acc[k] = 0;
 			tilePhase<T, D, K>(cx, B, l0, N, A, act, fs, acc,
 				[&](int, int64_t o, int n, const T (&y)[4], const T (&)[4]) { put(t + o, n, y); },
 				[&](int k, int64_t, int, const T (&y)[4], const T (&f)[4], double (&ac)[3 * K]) {
@@ -476,7 +469,6 @@ __global__ void __launch_bounds__(PHB_TILE, 2) kBicgPersistent(Dom<double, D> do
 						ac[3 * k + 2] = fma(double(f[i]), double(f[i]), ac[3 * k + 2]);
 					}
 				});
-			blockSumTo<3 * K>(acc, pp + (size_t)tile * 3 * K);
 		});
 		if (!gridBarrier(ctrl)) return;
 		reduceSystems<K, 3, -1>(dom.ninst, pp, sst, range, [&](SysState &s, int in, const double *red, double) {
@@ -492,10 +484,7 @@ __global__ void __launch_bounds__(PHB_TILE, 2) kBicgPersistent(Dom<double, D> do
 		});
 		// x += alpha p + omega s, r = s - omega t, (r0, r), (r, r)
 		pp = partial + (size_t)(ph++ & 1) * half;
-		cx.tiles([&](int tile, const BlockTab &B, int l0) {
-			double acc[2 * K];
-#pragma unroll
-			for (int k = 0; k < 2 * K; ++k) acc[k] = 0;
+		cx.template tileSums<2 * K>(pp, ws, [&](const BlockTab &B, int l0, double (&acc)[2 * K]) {
 			const int l = l0 + 4 * int(threadIdx.x);
 			const int n = max(0, min(4, B.cells() - l));
 			const bool al = cx.rows4(B) && n == 4;
@@ -532,7 +521,6 @@ __global__ void __launch_bounds__(PHB_TILE, 2) kBicgPersistent(Dom<double, D> do
 				st4(x + o, n, al, xv);
 				st4(r + o, n, al, rv);
 			}
-			blockSumTo<2 * K>(acc, pp + (size_t)tile * 2 * K);
 		});
 		if (!gridBarrier(ctrl)) return;
 		running = reduceSystems<K, 2, -1>(dom.ninst, pp, sst, range, [&](SysState &s, int in, const double *red, double) {
@@ -617,7 +605,7 @@ int launchPersistent(const phb_domain *dom, const phb_solve *sv, cudaStream_t s,
 	cfg.attrs = attr;
 	cfg.numAttrs = 1;
 	auto grid = [&](const void *kern) -> int {
-		if (smem > 24 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+		if (smem > 16 * 1024) (void)allowSmem(kern);
 		int perSM = 0;
 		if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, PHB_TILE, smem) != cudaSuccess || perSM < 1) perSM = 1;
 		if (sv->ctas_per_sm > 0) perSM = std::min(perSM, sv->ctas_per_sm); // a tuned, smaller grid

@@ -465,25 +465,45 @@ __device__ __forceinline__ bool gridBarrier(Control *ctrl, unsigned int spinLimi
 	return sOk;
 }
 
-// Block sum of NV values written to dst[0..NV) by the first threads.
+// Sums of NV values over each tile (item) that a CTA visits in a phase, without a CTA barrier per
+// tile: the warps leave their sums in shared memory and stream on, and one barrier for TILE_SUMS
+// tiles lets a thread per value add the warps up, in warp order (the order of storePartials). A barrier
+// per tile made the warps of a CTA wait for the slowest load of every tile: on grids of several
+// tiles per CTA a quarter of the stall cycles.
+constexpr int TILE_SUMS = 8;
 template <int NV>
-__device__ __forceinline__ void blockSumTo(double (&v)[NV], double *dst) {
-	__shared__ double sm[NV][NWARPS];
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+struct TileSums {
+	double (*ws)[NV][NWARPS]; // [TILE_SUMS], shared memory
+	double *dst;              // the phase's partials, [item][NV]
+	int k;                    // items visited so far
+	__device__ __forceinline__ void add(double (&v)[NV]) {
+		const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-	for (int q = 0; q < NV; ++q) {
-		const double s = warpSum(v[q]);
-		if (lane == 0) sm[q][warp] = s;
+		for (int q = 0; q < NV; ++q) {
+			const double s = warpSum(v[q]);
+			if (lane == 0) ws[k % TILE_SUMS][q][warp] = s;
+		}
 	}
-	__syncthreads();
-	if (threadIdx.x < NV) {
-		double s = 0;
+	// after every item, whether it added its sums or was left out (all threads)
+	__device__ __forceinline__ void next() {
+		if (++k % TILE_SUMS == 0) flush(TILE_SUMS);
+	}
+	// after the last item
+	__device__ __forceinline__ void finish() {
+		if (k % TILE_SUMS) flush(k % TILE_SUMS);
+	}
+	__device__ __forceinline__ void flush(int n) {
+		__syncthreads();
+		for (int i = threadIdx.x; i < n * NV; i += blockDim.x) {
+			const int slot = i / NV, q = i - slot * NV;
+			double s = 0;
 #pragma unroll
-		for (int w = 0; w < NWARPS; ++w) s += sm[threadIdx.x][w];
-		dst[threadIdx.x] = s;
+			for (int w = 0; w < NWARPS; ++w) s += ws[slot][q][w];
+			dst[(size_t)(blockIdx.x + (k - n + slot) * gridDim.x) * NV + q] = s;
+		}
+		__syncthreads();
 	}
-	__syncthreads();
-}
+};
 
 // block tables -----------------------------------------------------------------------------
 // What the phases of a persistent kernel need of one block of one level, kept in shared memory for
@@ -752,6 +772,18 @@ __device__ __forceinline__ SysState initialState(const phb_tolerance &tol, int s
 	z.restart = 1;
 	z.bestIt = -1;
 	return z;
+}
+
+// Lets launches of `kern` ask for as much dynamic shared memory as the device has (always the same
+// limit, so that threads launching with different sizes do not undo each other's).
+inline cudaError_t allowSmem(const void *kern) {
+	cudaFuncAttributes at;
+	int dev = 0, optin = 0;
+	cudaError_t e = cudaFuncGetAttributes(&at, kern);
+	if (e == cudaSuccess) e = cudaGetDevice(&dev);
+	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+	if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)at.sharedSizeBytes);
+	return e;
 }
 
 // kInit launched on `s`: the initial state of the nsys systems of a solve (krylov.cu)
