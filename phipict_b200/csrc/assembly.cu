@@ -12,9 +12,16 @@
 #include "phb_launch.cuh"
 #include "phb_nonortho.cuh"
 #include "phb_upwind.cuh"
+#include "phb_faces.cuh"
 #include <initializer_list>
 
 namespace phb {
+
+// CTAs per SM that the register budget of the branch-free kernels allows: a 3D float64 cell has 55
+// loads in flight (128 registers; at three CTAs the matrix on 192^3 took 484 instead of 351 us), the
+// others fit 85 (1999x1501 float32: 69 instead of 83 us).
+template <typename S, int D>
+constexpr int asmCtas() { return sizeof(S) == 8 && D == 3 ? 2 : 3; }
 
 // PISO_build_matrix (piso/advection.cu:27-305): implicit Euler advection-diffusion row
 // divided by the cell determinant; Adiag = its diagonal. SCALAR: the matrix of passive-scalar
@@ -105,6 +112,73 @@ __global__ void __launch_bounds__(PHB_TILE) kAdvectionMatrix(Dom<S, D> dom, cons
 	}
 }
 
+// The central, orthogonal matrix (no cross terms, no upwinding): same arithmetic, all loads of a
+// cell in flight together, several tiles per CTA (phb_faces.cuh). 192^3 float64: 522 -> 347 us (196 B
+// a cell, 0.62 of HBM counting the ten transform values it uses), 1999x1501 float32: 101 -> 66 us.
+template <typename S, int D, bool SCALAR>
+__global__ void __launch_bounds__(PHB_TILE, (asmCtas<S, D>())) kAdvectionMatrixCentral(Dom<S, D> dom, const S *__restrict__ u, S *__restrict__ C,
+		S *__restrict__ Adiag, float *__restrict__ Clo, ScalarView sv, int channel) {
+	__shared__ int32_t sB[PHB_BREC];
+	__shared__ FaceMap sF[6];
+	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
+		constexpr bool SAME = decltype(aligned)::value;
+		const int inst = sB[B_INST];
+		const S dt = S(dom.dt[inst]);
+		const S nu = SCALAR ? S(scalarNu(sv, channel, dom.nu[inst])) : S(dom.nu[inst]);
+		const int64_t N = dom.ncells;
+		const Comps<S, D> uc(sB, u);
+		for (int j_ = 0; j_ < CPT; ++j_) {
+			Cell c;
+			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
+			const Faces<D> n = cellFaces<D>(sB, sF, c);
+			S alphaN[2 * D], alphaP[D], fl[2 * D];
+#pragma unroll
+			for (int f = 0; f < 2 * D; ++f) alphaN[f] = alphaAt<S, D>(dom, n.om[f], SAME ? f >> 1 : n.comp[f]);
+#pragma unroll
+			for (int d = 0; d < D; ++d) alphaP[d] = alphaAt<S, D>(dom, c.mi, d);
+			cellFluxes<S, D, SAME>(dom, c, n, uc, fl);
+			const S det = detAt<S, D>(dom, c.mi);
+			S slip[2 * D];
+#pragma unroll
+			for (int f = 0; f < 2 * D; ++f) slip[f] = S(1);
+			if (n.fixed) {
+#pragma unroll
+				for (int f = 0; f < 2 * D; ++f) {
+					if (!((n.fixed >> f) & 1)) continue;
+					const int fid = fRec(sB, f)[5];
+					const int type = SCALAR ? int(sv.types[(int64_t)fid * sv.channels + channel]) : dom.fix(fid)[F_VELTYPE];
+					slip[f] = type == 0 ? S(0) : S(1);
+				}
+			}
+			S diag = det / dt;
+			S rv[2 * D + 1];
+#pragma unroll
+			for (int f = 0; f < 2 * D; ++f) {
+				const int dim = f >> 1;
+				const S half = S(0.5) * (((f & 1) ? S(1) : S(-1)) * fl[f]);
+				const S coeff = (alphaP[dim] * nu + alphaN[f] * nu) * S(0.5);
+				rv[f + 1] = 0;
+				if (!((n.fixed >> f) & 1)) {
+					diag += half;
+					rv[f + 1] += half;
+					diag += coeff;
+					rv[f + 1] -= coeff;
+				} else {
+					diag += (S(1) - slip[f]) * S(2) * nu * alphaP[dim];
+				}
+			}
+			rv[0] = diag;
+#pragma unroll
+			for (int s = 0; s < 2 * D + 1; ++s) {
+				const S v = rv[s] / det;
+				C[s * N + c.g] = v;
+				if (Clo) Clo[s * N + c.g] = float(v);
+			}
+			Adiag[c.g] = rv[0] / det;
+		}
+	});
+}
+
 // boundary source of the momentum equation at fixed faces (advection.cu:834-866, the same
 // terms as pressure.cu:404-432): -u_b F_b + 2 nu alpha u_b (no-slip faces)
 template <typename S, int D>
@@ -132,10 +206,10 @@ __device__ __forceinline__ S sourceAt(const Cell &c, const S *__restrict__ src, 
 	return S(0);
 }
 
-// kPISO_build_advection_RHS (advection.cu:800-954), no pressure gradient. A thread takes four
+// kPISO_build_advection_RHS (advection.cu:800-954), no pressure gradient, LINEAR_UPWIND. A thread takes four
 // consecutive cells (Quad): their transforms, velocities and sources load as vectors; the
 // fixed-face sources and the LINEAR_UPWIND correction are added per cell where they apply.
-template <typename S, int D, bool UPW>
+template <typename S, int D>
 __global__ void __launch_bounds__(PHB_TILE, sizeof(S) == 8 ? 2 : 3) kAdvectionRhs(Dom<S, D> dom, const S *__restrict__ u, const S *__restrict__ src,
 		int srcMode, S *__restrict__ rhs) {
 	__shared__ int32_t sB[PHB_BREC];
@@ -150,8 +224,6 @@ __global__ void __launch_bounds__(PHB_TILE, sizeof(S) == 8 ? 2 : 3) kAdvectionRh
 	const int64_t mi0 = sB[B_METOFF] + q.l;
 	S det[4];
 	ld4(dom.met + Tr<D>::DET * dom.ms + mi0, q.n, metAligned(dom, q, mi0), det);
-	// cells with a fixed face, or every cell with LINEAR_UPWIND, take the per-cell terms
-	const bool perCell = UPW || !q.fast || q.p[0] == 0 || q.p[0] + 3 == sB[B_NX] - 1;
 #pragma unroll
 	for (int dim = 0; dim < D; ++dim) {
 		const int64_t o = vidx<D>(q.B, q.g, dim);
@@ -159,19 +231,15 @@ __global__ void __launch_bounds__(PHB_TILE, sizeof(S) == 8 ? 2 : 3) kAdvectionRh
 		ld4(u + o, q.n, q.al, uv);
 #pragma unroll
 		for (int i = 0; i < 4; ++i) r[i] = det[i] * uv[i] / dt;
-		if (perCell) {
 #pragma unroll
-			for (int i = 0; i < 4; ++i) {
-				if (i >= q.n) break;
-				Cell c;
-				quadCell<D>(q, i, c);
-				r[i] += boundarySource<S, D>(dom, c, dim, nu);
-				if constexpr (UPW) {
-					S fl[2 * D];
-					faceFluxes<S, D>(dom, c, u, fl);
-					upwindCorrection<S, D>(c, fl, [&](int64_t g) { return u[vidx<D>(c.B, g, dim)]; }, r[i]);
-				}
-			}
+		for (int i = 0; i < 4; ++i) {
+			if (i >= q.n) break;
+			Cell c;
+			quadCell<D>(q, i, c);
+			r[i] += boundarySource<S, D>(dom, c, dim, nu);
+			S fl[2 * D];
+			faceFluxes<S, D>(dom, c, u, fl);
+			upwindCorrection<S, D>(c, fl, [&](int64_t g) { return u[vidx<D>(c.B, g, dim)]; }, r[i]);
 		}
 		S sv[4] = {0, 0, 0, 0};
 		if (srcMode == 1) {
@@ -185,6 +253,48 @@ __global__ void __launch_bounds__(PHB_TILE, sizeof(S) == 8 ? 2 : 3) kAdvectionRh
 		for (int i = 0; i < 4; ++i) r[i] = r[i] / det[i] + sv[i];
 		st4(rhs + o, q.n, q.al, r);
 	}
+}
+
+// The same for the central scheme, one cell at a time: a streaming kernel, its few cells on fixed
+// faces corrected after the loads. 192^3 float64: 245 us with a CTA per tile, 171 with several.
+template <typename S, int D>
+__global__ void __launch_bounds__(PHB_TILE, 4) kAdvectionRhsCentral(Dom<S, D> dom, const S *__restrict__ u, const S *__restrict__ src,
+		int srcMode, S *__restrict__ rhs) {
+	__shared__ int32_t sB[PHB_BREC];
+	__shared__ FaceMap sF[6];
+	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
+		constexpr bool SAME = decltype(aligned)::value;
+		const int inst = sB[B_INST];
+		const S dt = S(dom.dt[inst]);
+		const S nu = S(dom.nu[inst]);
+#pragma unroll 2
+		const Comps<S, D> uc(sB, u);
+		for (int j_ = 0; j_ < CPT; ++j_) {
+			Cell c;
+			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
+			S uv[D], sv[D], bs[D];
+#pragma unroll
+			for (int d = 0; d < D; ++d) {
+				uv[d] = uc.c[d][c.g];
+				sv[d] = sourceAt<S, D>(c, src, srcMode, d);
+				bs[d] = 0;
+			}
+			const S det = detAt<S, D>(dom, c.mi);
+			bool fixed = false;
+#pragma unroll
+			for (int f = 0; f < 2 * D; ++f) fixed = fixed || (atBound(sB, f, c.p) && !sF[f].open);
+			if (fixed) {
+#pragma unroll
+				for (int d = 0; d < D; ++d) bs[d] = boundarySource<S, D>(dom, c, d, nu);
+			}
+#pragma unroll
+			for (int d = 0; d < D; ++d) {
+				S r = det * uv[d] / dt;
+				r += bs[d];
+				rhs[vidx<D>(sB, c.g, d)] = r / det + sv[d];
+			}
+		}
+	});
 }
 
 // kPISO_build_scalar_advection_RHS (advection.cu:545-698), CENTRAL, orthogonal:
@@ -344,6 +454,50 @@ __global__ void __launch_bounds__(PHB_TILE) kLaplaceMatrix(Dom<S, D> dom, const 
 	}
 }
 
+// The pressure matrix without cross terms: same arithmetic, all loads of a cell in flight together.
+// 192^3 float64: 261 -> 229 us (0.69 of HBM).
+template <typename S, int D>
+__global__ void __launch_bounds__(PHB_TILE, 3) kPressureMatrix(Dom<S, D> dom, const S *__restrict__ Adiag, S *__restrict__ P,
+		float *__restrict__ Plo) {
+	__shared__ int32_t sB[PHB_BREC];
+	__shared__ FaceMap sF[6];
+	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
+		constexpr bool SAME = decltype(aligned)::value;
+		const int64_t N = dom.ncells;
+		for (int j_ = 0; j_ < CPT; ++j_) {
+			Cell c;
+			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
+			const Faces<D> n = cellFaces<D>(sB, sF, c);
+			S alphaN[2 * D], alphaP[D], aN[2 * D];
+#pragma unroll
+			for (int f = 0; f < 2 * D; ++f) {
+				alphaN[f] = alphaAt<S, D>(dom, n.om[f], SAME ? f >> 1 : n.comp[f]);
+				aN[f] = Adiag[n.o[f]];
+			}
+#pragma unroll
+			for (int d = 0; d < D; ++d) alphaP[d] = alphaAt<S, D>(dom, c.mi, d);
+			const S raP = S(1) / Adiag[c.g];
+			S rv[2 * D + 1];
+			rv[0] = 0;
+#pragma unroll
+			for (int f = 0; f < 2 * D; ++f) {
+				const S raN = S(1) / aN[f];
+				const S coeff = S(0.5) * (alphaP[f >> 1] * raP + alphaN[f] * raN);
+				rv[f + 1] = 0;
+				if (!((n.fixed >> f) & 1)) {
+					rv[0] -= coeff;
+					rv[f + 1] += coeff;
+				}
+			}
+#pragma unroll
+			for (int s = 0; s < 2 * D + 1; ++s) {
+				P[s * N + c.g] = rv[s];
+				if (Plo) Plo[s * N + c.g] = float(rv[s]);
+			}
+		}
+	});
+}
+
 // The cold paths of kPressureRhs: H of cell i of a quad off the fast path, resolving each
 // face ...
 template <typename S, int D>
@@ -371,42 +525,39 @@ __device__ __forceinline__ CompSums<S, D> hbyaSlowH(const Dom<S, D> &dom, const 
 	return h;
 }
 // ... and the source of cell i with its fixed faces and the deferred LINEAR_UPWIND correction
-template <typename S, int D, bool UPW>
+template <typename S, int D>
 __device__ __forceinline__ S hbyaCellSource(const Dom<S, D> &dom, const Quad &q, int i, int dim, S nu, S det, S src, const S *__restrict__ u) {
 	Cell c;
 	quadCell<D>(q, i, c);
 	S Ssum = boundarySource<S, D>(dom, c, dim, nu);
 	Ssum /= det;
 	Ssum += src;
-	if constexpr (UPW) {
-		// HbyA repeats the predictor's deferred correction (pressure.cu:474-515)
-		S fl[2 * D];
-		faceFluxes<S, D>(dom, c, u, fl);
-		S corr = 0;
-		upwindCorrection<S, D>(c, fl, [&](int64_t g) { return u[vidx<D>(c.B, g, dim)]; }, corr);
-		Ssum += corr / det;
-	}
+	// HbyA repeats the predictor's deferred correction (pressure.cu:474-515)
+	S fl[2 * D];
+	faceFluxes<S, D>(dom, c, u, fl);
+	S corr = 0;
+	upwindCorrection<S, D>(c, fl, [&](int64_t g) { return u[vidx<D>(c.B, g, dim)]; }, corr);
+	Ssum += corr / det;
 	return Ssum;
 }
 
-// Out-of-line calls of the two: in 3D the inlined cold paths make the kernel large enough to
-// stall on instruction fetch (measured: HbyA on 256^3 at 0.38 of HBM out of line against 0.34
-// inline), in 2D inlining is faster (0.66 against 0.55 on 4096^2).
+// Out-of-line calls of the two: in 3D the inlined paths make the kernel large enough to stall on
+// instruction fetch, in 2D inlining is faster.
 template <typename S, int D>
 __device__ __noinline__ CompSums<S, D> hbyaSlowHCall(const Dom<S, D> &dom, const Quad &q, int i, const S *__restrict__ C,
 		const S *__restrict__ ustar) {
 	return hbyaSlowH<S, D>(dom, q, i, C, ustar);
 }
-template <typename S, int D, bool UPW>
+template <typename S, int D>
 __device__ __noinline__ S hbyaCellSourceCall(const Dom<S, D> &dom, const Quad &q, int i, int dim, S nu, S det, S src,
 		const S *__restrict__ u) {
-	return hbyaCellSource<S, D, UPW>(dom, q, i, dim, nu, det, src, u);
+	return hbyaCellSource<S, D>(dom, q, i, dim, nu, det, src, u);
 }
 
-// PISO_build_pressure_rhs (pressure.cu:350-521): HbyA = (u/dt - H(u*) + S)/A per component,
+// PISO_build_pressure_rhs (pressure.cu:350-521) with LINEAR_UPWIND: HbyA = (u/dt - H(u*) + S)/A per component,
 // four consecutive cells per thread. H sums the stencil's face slots in face order for every
 // component at once, so that a slot's four values are loaded once and dropped.
-template <typename S, int D, bool UPW>
+template <typename S, int D>
 __global__ void __launch_bounds__(PHB_TILE, sizeof(S) == 8 ? 2 : 3) kPressureRhs(Dom<S, D> dom, const S *__restrict__ C, const S *__restrict__ Adiag,
 		const S *__restrict__ u, const S *__restrict__ ustar, const S *__restrict__ src, int srcMode, S *__restrict__ hbya) {
 	__shared__ int32_t sB[PHB_BREC];
@@ -485,7 +636,6 @@ __global__ void __launch_bounds__(PHB_TILE, sizeof(S) == 8 ? 2 : 3) kPressureRhs
 	S a[4], det[4];
 	ld4(Adiag + q.g, q.n, q.al, a);
 	ld4(dom.met + Tr<D>::DET * dom.ms + mi0, q.n, metAligned(dom, q, mi0), det);
-	const bool perCell = UPW || !q.fast || q.p[0] == 0 || q.p[0] + 3 == sB[B_NX] - 1;
 #pragma unroll
 	for (int dim = 0; dim < D; ++dim) {
 		const int64_t o = o0 + dim * cs;
@@ -502,12 +652,9 @@ __global__ void __launch_bounds__(PHB_TILE, sizeof(S) == 8 ? 2 : 3) kPressureRhs
 #pragma unroll
 		for (int i = 0; i < 4; ++i) {
 			S Ssum = 0;
-			if (perCell && i < q.n) {
-				Ssum = D > 2 ? hbyaCellSourceCall<S, D, UPW>(dom, q, i, dim, nu, det[i], sv[i], u)
-				             : hbyaCellSource<S, D, UPW>(dom, q, i, dim, nu, det[i], sv[i], u);
-			} else {
-				Ssum /= det[i];
-				Ssum += sv[i];
+			if (i < q.n) {
+				Ssum = D > 2 ? hbyaCellSourceCall<S, D>(dom, q, i, dim, nu, det[i], sv[i], u)
+				             : hbyaCellSource<S, D>(dom, q, i, dim, nu, det[i], sv[i], u);
 			}
 			out[i] = (S(1) / a[i]) * (uv[i] / dt - H[dim][i] + Ssum);
 		}
@@ -515,67 +662,113 @@ __global__ void __launch_bounds__(PHB_TILE, sizeof(S) == 8 ? 2 : 3) kPressureRhs
 	}
 }
 
-// k_computePressureRHSdivergenceFromFlux (pressure.cu:756-801), no face transforms
+// HbyA of the central scheme, one cell at a time with all its loads in flight together: the row form
+// above resolves the faces of the quads that touch one (192^3 float64: 585 us in that form, 408 here).
 template <typename S, int D>
-__global__ void __launch_bounds__(PHB_TILE) kDivergence(Dom<S, D> dom, const S *__restrict__ field, S *__restrict__ div) {
+__global__ void __launch_bounds__(PHB_TILE, 3) kPressureRhsCentral(Dom<S, D> dom, const S *__restrict__ C, const S *__restrict__ Adiag,
+		const S *__restrict__ u, const S *__restrict__ ustar, const S *__restrict__ src, int srcMode, S *__restrict__ hbya) {
 	__shared__ int32_t sB[PHB_BREC];
-	int l0_, nc_;
-	loadTile<S, D>(dom, sB, l0_, nc_);
-	for (int j_ = 0; j_ < CPT; ++j_) {
-	Cell c;
-	if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
-	S fl[2 * D];
-	faceFluxes<S, D>(dom, c, field, fl);
-	S dv = 0;
+	__shared__ FaceMap sF[6];
+	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
+		constexpr bool SAME = decltype(aligned)::value;
+		const int inst = sB[B_INST];
+		const S dt = S(dom.dt[inst]);
+		const S nu = S(dom.nu[inst]);
+		const int64_t N = dom.ncells;
+		const Comps<S, D> usc(sB, ustar), uc(sB, u);
+		for (int j_ = 0; j_ < CPT; ++j_) {
+			Cell c;
+			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
+			const Faces<D> n = cellFaces<D>(sB, sF, c);
+			S cv[2 * D], H[D], uv[D], sv[D];
 #pragma unroll
-	for (int d = 0; d < D; ++d) dv += fl[d * 2 + 1] - fl[d * 2];
-	div[c.g] = dv;
-	}
+			for (int f = 0; f < 2 * D; ++f) cv[f] = C[(f + 1) * N + c.g];
+#pragma unroll
+			for (int d = 0; d < D; ++d) {
+				S v[2 * D];
+#pragma unroll
+				for (int f = 0; f < 2 * D; ++f) v[f] = usc.c[d][n.o[f]];
+				H[d] = 0;
+				// no term without neighbour, nor on a periodic axis one cell wide (the cell itself)
+#pragma unroll
+				for (int f = 0; f < 2 * D; ++f) H[d] = fma(cv[f], n.o[f] == c.g ? S(0) : v[f], H[d]);
+				uv[d] = uc.c[d][c.g];
+				sv[d] = sourceAt<S, D>(c, src, srcMode, d);
+			}
+			const S a = Adiag[c.g], det = detAt<S, D>(dom, c.mi);
+			S bs[D];
+#pragma unroll
+			for (int d = 0; d < D; ++d) bs[d] = 0;
+			if (n.fixed) {
+#pragma unroll
+				for (int d = 0; d < D; ++d) bs[d] = boundarySource<S, D>(dom, c, d, nu);
+			}
+#pragma unroll
+			for (int d = 0; d < D; ++d) {
+				S Ssum = bs[d] / det;
+				Ssum += sv[d];
+				hbya[vidx<D>(sB, c.g, d)] = (S(1) / a) * (uv[d] / dt - H[d] + Ssum);
+			}
+		}
+	});
 }
 
-// getPressureAtWithBounds for the +-1 neighbours (nonortho_laplace.cuh:302-381)
+// k_computePressureRHSdivergenceFromFlux (pressure.cu:756-801), no face transforms (192^3 float64:
+// 275 -> 229 us, 0.54 of HBM: 55 loads a cell, most of them L1 hits, bound the issue)
 template <typename S, int D>
-__device__ __forceinline__ S scalarAcross(const Dom<S, D> &dom, const Cell &c, int f, const S *__restrict__ p) {
-	if (atBound(c.B, f, c.p) && fType(c.B, f) == FT_FIXED) return p[c.g];
-	return p[neighbor<S, D>(dom, c, f).g];
+__global__ void __launch_bounds__(PHB_TILE, (asmCtas<S, D>())) kDivergence(Dom<S, D> dom, const S *__restrict__ field, S *__restrict__ div) {
+	__shared__ int32_t sB[PHB_BREC];
+	__shared__ FaceMap sF[6];
+	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
+		constexpr bool SAME = decltype(aligned)::value;
+		const Comps<S, D> fc(sB, field);
+		for (int j_ = 0; j_ < CPT; ++j_) {
+			Cell c;
+			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
+			S fl[2 * D];
+			cellFluxes<S, D, SAME>(dom, c, cellFaces<D>(sB, sF, c), fc, fl);
+			S dv = 0;
+#pragma unroll
+			for (int d = 0; d < D; ++d) dv += fl[d * 2 + 1] - fl[d * 2];
+			div[c.g] = dv;
+		}
+	});
 }
 
 // PISO_update_velocity, version 1 (velocity_correction.cu:27-60) with the finite
 // difference gradient of getPressureGradient (piso/device/velocity.cuh:347-378)
 template <typename S, int D>
-__global__ void __launch_bounds__(PHB_TILE) kCorrectVelocity(Dom<S, D> dom, const S *__restrict__ p, const S *__restrict__ hbya,
+__global__ void __launch_bounds__(PHB_TILE, 4) kCorrectVelocity(Dom<S, D> dom, const S *__restrict__ p, const S *__restrict__ hbya,
 		const S *__restrict__ Adiag, S *__restrict__ u) {
 	__shared__ int32_t sB[PHB_BREC];
-	int l0_, nc_;
-	loadTile<S, D>(dom, sB, l0_, nc_);
-	for (int j_ = 0; j_ < CPT; ++j_) {
-	Cell c;
-	if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
-	const S rDiag = S(1) / Adiag[c.g];
-	S gr[D];
+	__shared__ FaceMap sF[6];
+	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
+		constexpr bool SAME = decltype(aligned)::value;
+		for (int j_ = 0; j_ < CPT; ++j_) {
+			Cell c;
+			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
+			const Faces<D> n = cellFaces<D>(sB, sF, c);
+			S pn[2 * D], hv[D];
 #pragma unroll
-	for (int dim = 0; dim < D; ++dim) {
-		S fac = 0.5;
-		const bool lowFixed = c.p[dim] == 0 && fType(c.B, dim * 2) == FT_FIXED;
-		const bool upFixed = c.p[dim] == c.B[B_NX + dim] - 1 && fType(c.B, dim * 2 + 1) == FT_FIXED;
-		if (lowFixed || upFixed) fac = 1;
-		const S valN = lowFixed ? p[c.g] : scalarAcross<S, D>(dom, c, dim * 2, p);
-		const S valP = upFixed ? p[c.g] : scalarAcross<S, D>(dom, c, dim * 2 + 1, p);
-		gr[dim] = (valP - valN) * fac;
-	}
-	S grad[D];
+			for (int f = 0; f < 2 * D; ++f) pn[f] = p[n.o[f]]; // a fixed face: the cell's own value
 #pragma unroll
-	for (int k = 0; k < D; ++k) grad[k] = 0;
+			for (int d = 0; d < D; ++d) hv[d] = hbya[vidx<D>(sB, c.g, d)];
+			const S rDiag = S(1) / Adiag[c.g];
+			S gr[D], grad[D];
 #pragma unroll
-	for (int r = 0; r < D; ++r)
+			for (int d = 0; d < D; ++d) {
+				const S fac = (n.fixed >> (2 * d)) & 3 ? S(1) : S(0.5);
+				gr[d] = (pn[2 * d + 1] - pn[2 * d]) * fac;
+				grad[d] = 0;
+			}
 #pragma unroll
-		for (int k = 0; k < D; ++k) grad[k] += dom.m(Tr<D>::MINV + r * D + k, c.mi) * gr[r];
+			for (int r = 0; r < D; ++r)
 #pragma unroll
-	for (int d = 0; d < D; ++d) {
-		const int64_t o = vidx<D>(c.B, c.g, d);
-		u[o] = -rDiag * grad[d] + hbya[o];
-	}
-	}
+				for (int k = 0; k < D; ++k) grad[k] += dom.m(Tr<D>::MINV + r * D + k, c.mi) * gr[r];
+#pragma unroll
+			for (int d = 0; d < D; ++d) u[vidx<D>(sB, c.g, d)] = -rDiag * grad[d] + hv[d];
+		}
+	});
 }
 
 // u x e_b at a cell (simulation/mhd.py:276-355): 2D velocities are lifted to 3D
@@ -589,49 +782,26 @@ __device__ __forceinline__ void uCrossB(const int32_t *B, int64_t g, const S *__
 	out[2] = u0 * e1 - u1 * e0;
 }
 
-// u x e_b fused with k_computeEpotRHS (mhd/potential.cu:273-323) and its face fluxes
-// computeEpotFluxesNDLoop (discretization.cuh:856-912)
+// Corrections of the potential right-hand side on fixed faces: no current through insulating and
+// thin walls, the cell's own flux elsewhere (computeEpotFluxesNDLoop, discretization.cuh:856-912) ...
 template <typename S, int D>
-__global__ void __launch_bounds__(PHB_TILE) kUxbEpotRhs(Dom<S, D> dom, const S *__restrict__ u, const double *__restrict__ eb,
-		S *__restrict__ uxb, S *__restrict__ rhs) {
-	__shared__ int32_t sB[PHB_BREC];
-	int l0_, nc_;
-	loadTile<S, D>(dom, sB, l0_, nc_);
-	for (int j_ = 0; j_ < CPT; ++j_) {
-	Cell c;
-	if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
-	const double *e = eb + 3 * c.B[B_INST];
-	S x[3];
-	uCrossB<S, D>(c.B, c.g, u, e, x);
-#pragma unroll
-	for (int k = 0; k < 3; ++k) uxb[vidx3(c.B, c.g, k)] = x[k];
-	S fl[2 * D];
-#pragma unroll
-	for (int dim = 0; dim < D; ++dim) {
-		const S velC = contraVec<S, D>(dom, c.mi, dim, x);
-#pragma unroll
-		for (int up = 0; up < 2; ++up) {
-			const int f = dim * 2 + up;
-			if (atBound(c.B, f, c.p) && fType(c.B, f) == FT_FIXED) {
-				const int32_t *FR = dom.fix(fRec(c.B, f)[5]);
-				const int bc = potBC(dom.fmask, FR, faceCell(c.B, f, c.p));
-				fl[f] = (bc == PB_INSULATING || bc == PB_THIN_WALL) ? S(0) : velC;
-			} else {
-				const Nbr n = neighbor<S, D>(dom, c, f);
-				S xn[3];
-				uCrossB<S, D>(n.B, n.g, u, e, xn);
-				S velN = contraVec<S, D>(dom, n.mi, n.comp, xn);
-				if (n.flip) velN = -velN;
-				fl[f] = (velN + velC) * S(0.5);
-			}
-		}
-	}
-	S dv = 0;
-#pragma unroll
-	for (int d = 0; d < D; ++d) dv += fl[d * 2 + 1] - fl[d * 2];
+__device__ __forceinline__ void epotFixedFluxes(const Dom<S, D> &dom, const Cell &c, unsigned int fixed, const S (&vC)[D], S (&fl)[2 * D]) {
+	if (!fixed) return;
 #pragma unroll
 	for (int f = 0; f < 2 * D; ++f) {
-		if (!atBound(c.B, f, c.p) || fType(c.B, f) != FT_FIXED) continue;
+		if (!((fixed >> f) & 1)) continue;
+		const int32_t *FR = dom.fix(fRec(c.B, f)[5]);
+		const int bc = potBC(dom.fmask, FR, faceCell(c.B, f, c.p));
+		fl[f] = (bc == PB_INSULATING || bc == PB_THIN_WALL) ? S(0) : vC[f >> 1];
+	}
+}
+// ... and the prescribed values of Dirichlet faces
+template <typename S, int D>
+__device__ __forceinline__ void epotDirichlet(const Dom<S, D> &dom, const Cell &c, unsigned int fixed, S &dv) {
+	if (!fixed) return;
+#pragma unroll
+	for (int f = 0; f < 2 * D; ++f) {
+		if (!((fixed >> f) & 1)) continue;
 		const int32_t *FR = dom.fix(fRec(c.B, f)[5]);
 		const int fc = faceCell(c.B, f, c.p);
 		if (potBC(dom.fmask, FR, fc) != PB_DIRICHLET) continue;
@@ -639,53 +809,72 @@ __global__ void __launch_bounds__(PHB_TILE) kUxbEpotRhs(Dom<S, D> dom, const S *
 		if (gv == S(0)) continue;
 		dv -= alphaAt<S, D>(dom, c.mi, f >> 1) * gv;
 	}
-	rhs[c.g] = dv;
-	}
+}
+
+// u x e_b fused with k_computeEpotRHS (mhd/potential.cu:273-323)
+template <typename S, int D>
+__global__ void __launch_bounds__(PHB_TILE, (asmCtas<S, D>())) kUxbEpotRhs(Dom<S, D> dom, const S *__restrict__ u, const double *__restrict__ eb,
+		S *__restrict__ uxb, S *__restrict__ rhs) {
+	__shared__ int32_t sB[PHB_BREC];
+	__shared__ FaceMap sF[6];
+	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
+		constexpr bool SAME = decltype(aligned)::value;
+		const double *e = eb + 3 * sB[B_INST];
+		for (int j_ = 0; j_ < CPT; ++j_) {
+			Cell c;
+			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
+			const Faces<D> n = cellFaces<D>(sB, sF, c);
+			S vN[2 * D], vC[D], x[3], fl[2 * D];
+#pragma unroll
+			for (int f = 0; f < 2 * D; ++f) {
+				S xn[3];
+				uCrossB<S, D>(c.B, n.o[f], u, e, xn);
+				vN[f] = contraVec<S, D>(dom, n.om[f], SAME ? f >> 1 : n.comp[f], xn);
+			}
+			uCrossB<S, D>(c.B, c.g, u, e, x);
+#pragma unroll
+			for (int d = 0; d < D; ++d) vC[d] = contraVec<S, D>(dom, c.mi, d, x);
+#pragma unroll
+			for (int k = 0; k < 3; ++k) uxb[vidx3(c.B, c.g, k)] = x[k];
+#pragma unroll
+			for (int f = 0; f < 2 * D; ++f) fl[f] = (((n.flip >> f) & 1 ? -vN[f] : vN[f]) + vC[f >> 1]) * S(0.5);
+			epotFixedFluxes<S, D>(dom, c, n.fixed, vC, fl);
+			S dv = 0;
+#pragma unroll
+			for (int d = 0; d < D; ++d) dv += fl[d * 2 + 1] - fl[d * 2];
+			epotDirichlet<S, D>(dom, c, n.fixed, dv);
+			rhs[c.g] = dv;
+		}
+	});
 }
 
 // k_computeEpotRHS (mhd/potential.cu:273-323) of a given in-plane field [inst][dims][cells]
 template <typename S, int D>
-__global__ void __launch_bounds__(PHB_TILE) kEpotRhs(Dom<S, D> dom, const S *__restrict__ field, S *__restrict__ rhs) {
+__global__ void __launch_bounds__(PHB_TILE, (asmCtas<S, D>())) kEpotRhs(Dom<S, D> dom, const S *__restrict__ field, S *__restrict__ rhs) {
 	__shared__ int32_t sB[PHB_BREC];
-	int l0_, nc_;
-	loadTile<S, D>(dom, sB, l0_, nc_);
-	for (int j_ = 0; j_ < CPT; ++j_) {
-	Cell c;
-	if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
-	S fl[2 * D];
+	__shared__ FaceMap sF[6];
+	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
+		constexpr bool SAME = decltype(aligned)::value;
+		const Comps<S, D> fc(sB, field);
+		for (int j_ = 0; j_ < CPT; ++j_) {
+			Cell c;
+			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
+			const Faces<D> n = cellFaces<D>(sB, sF, c);
+			S vN[2 * D], vC[D], fl[2 * D];
 #pragma unroll
-	for (int dim = 0; dim < D; ++dim) {
-		const S velC = contraAt<S, D>(dom, c.B, c.g, c.mi, dim, field);
+			for (int f = 0; f < 2 * D; ++f) vN[f] = contraComps<S, D>(dom, fc, n.o[f], n.om[f], SAME ? f >> 1 : n.comp[f]);
 #pragma unroll
-		for (int up = 0; up < 2; ++up) {
-			const int f = dim * 2 + up;
-			if (atBound(c.B, f, c.p) && fType(c.B, f) == FT_FIXED) {
-				const int32_t *FR = dom.fix(fRec(c.B, f)[5]);
-				const int bc = potBC(dom.fmask, FR, faceCell(c.B, f, c.p));
-				fl[f] = (bc == PB_INSULATING || bc == PB_THIN_WALL) ? S(0) : velC;
-			} else {
-				const Nbr n = neighbor<S, D>(dom, c, f);
-				S velN = contraAt<S, D>(dom, n.B, n.g, n.mi, n.comp, field);
-				if (n.flip) velN = -velN;
-				fl[f] = (velN + velC) * S(0.5);
-			}
+			for (int d = 0; d < D; ++d) vC[d] = contraComps<S, D>(dom, fc, c.g, c.mi, d);
+#pragma unroll
+			for (int f = 0; f < 2 * D; ++f) fl[f] = (((n.flip >> f) & 1 ? -vN[f] : vN[f]) + vC[f >> 1]) * S(0.5);
+			epotFixedFluxes<S, D>(dom, c, n.fixed, vC, fl);
+			S dv = 0;
+#pragma unroll
+			for (int d = 0; d < D; ++d) dv += fl[d * 2 + 1] - fl[d * 2];
+			epotDirichlet<S, D>(dom, c, n.fixed, dv);
+			rhs[c.g] = dv;
 		}
-	}
-	S dv = 0;
-#pragma unroll
-	for (int d = 0; d < D; ++d) dv += fl[d * 2 + 1] - fl[d * 2];
-#pragma unroll
-	for (int f = 0; f < 2 * D; ++f) {
-		if (!atBound(c.B, f, c.p) || fType(c.B, f) != FT_FIXED) continue;
-		const int32_t *FR = dom.fix(fRec(c.B, f)[5]);
-		const int fc = faceCell(c.B, f, c.p);
-		if (potBC(dom.fmask, FR, fc) != PB_DIRICHLET) continue;
-		const S gv = potValue<S, D>(dom, FR, fc);
-		if (gv == S(0)) continue;
-		dv -= alphaAt<S, D>(dom, c.mi, f >> 1) * gv;
-	}
-	rhs[c.g] = dv;
-	}
+	});
 }
 
 // computeCurrentDensityFaceBased (mhd/potential.cu:718-880) fused with the Lorentz force
@@ -848,6 +1037,7 @@ using namespace phb;
 		else return setError(PHB_ERR_ARG, "unsupported dims/dtype");                                \
 	} while (0)
 
+#define PHB_RESIDENT(DOM, KERN) tileGrid<KERN>((DOM)->ntiles), dim3(PHB_TILE), 0, (cudaStream_t)stream
 #define PHB_TILES(DOM) dim3((DOM)->ntiles), dim3(PHB_TILE), 0, (cudaStream_t)stream
 
 // The device view of a launch whose quad kernels may use vector loads: every field operand
@@ -871,7 +1061,11 @@ extern "C" int phb_advection_matrix(const phb_domain *dom, const void *u, void *
 		PHB_DISPATCH(dom, (kAdvectionMatrix<S, D, false, true><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)u, (S *)C, (S *)Adiag, C_lo)));
 		return checkLaunch("kAdvectionMatrix<non-orthogonal>");
 	}
-	PHB_DISPATCH(dom, kAdvectionMatrix<S, D><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)u, (S *)C, (S *)Adiag, C_lo));
+	if (dom->scheme == 0)
+		PHB_DISPATCH(dom, (kAdvectionMatrixCentral<S, D, false><<<PHB_RESIDENT(dom, (kAdvectionMatrixCentral<S, D, false>))>>>(Dom<S, D>(*dom), (const S *)u, (S *)C, (S *)Adiag, C_lo,
+			ScalarView{}, 0)));
+	else
+		PHB_DISPATCH(dom, kAdvectionMatrix<S, D><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)u, (S *)C, (S *)Adiag, C_lo));
 	return checkLaunch("kAdvectionMatrix");
 }
 extern "C" int phb_scalar_matrix(const phb_domain *dom, const void *u, const phb_scalar *sc, int channel, void *C, void *Adiag,
@@ -887,7 +1081,11 @@ extern "C" int phb_scalar_matrix(const phb_domain *dom, const void *u, const phb
 			channel)));
 		return checkLaunch("kAdvectionMatrix<scalar, non-orthogonal>");
 	}
-	PHB_DISPATCH(dom, kAdvectionMatrix<S, D, true><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)u, (S *)C, (S *)Adiag, C_lo, sv, channel));
+	if (dom->scheme == 0)
+		PHB_DISPATCH(dom, (kAdvectionMatrixCentral<S, D, true><<<PHB_RESIDENT(dom, (kAdvectionMatrixCentral<S, D, true>))>>>(Dom<S, D>(*dom), (const S *)u, (S *)C, (S *)Adiag, C_lo, sv,
+			channel)));
+	else
+		PHB_DISPATCH(dom, kAdvectionMatrix<S, D, true><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)u, (S *)C, (S *)Adiag, C_lo, sv, channel));
 	return checkLaunch("kAdvectionMatrix<scalar>");
 }
 extern "C" int phb_scalar_rhs(const phb_domain *dom, const void *phi, const void *u, const phb_scalar *sc, void *rhs, phb_stream stream) {
@@ -904,11 +1102,11 @@ extern "C" int phb_advection_rhs(const phb_domain *dom, const void *u, const voi
 	if (!dom || !u || !rhs || (src_mode != 0 && !src) || src_mode < 0 || src_mode > 2) return setError(PHB_ERR_ARG, "phb_advection_rhs: bad argument");
 	if (dom->ntiles == 0) return PHB_OK;
 	if (dom->scheme != 0)
-		PHB_DISPATCH(dom, (kAdvectionRhs<S, D, true><<<PHB_TILES(dom)>>>(quadView<S, D>(dom, {u, src, rhs}), (const S *)u, (const S *)src,
+		PHB_DISPATCH(dom, (kAdvectionRhs<S, D><<<PHB_TILES(dom)>>>(quadView<S, D>(dom, {u, src, rhs}), (const S *)u, (const S *)src,
 			src_mode, (S *)rhs)));
 	else
-		PHB_DISPATCH(dom, (kAdvectionRhs<S, D, false><<<PHB_TILES(dom)>>>(quadView<S, D>(dom, {u, src, rhs}), (const S *)u, (const S *)src,
-			src_mode, (S *)rhs)));
+		PHB_DISPATCH(dom, (kAdvectionRhsCentral<S, D><<<PHB_RESIDENT(dom, (kAdvectionRhsCentral<S, D>))>>>(Dom<S, D>(*dom), (const S *)u,
+			(const S *)src, src_mode, (S *)rhs)));
 	return checkLaunch("kAdvectionRhs");
 }
 extern "C" int phb_pressure_matrix(const phb_domain *dom, const void *Adiag, void *P, float *P_lo, phb_stream stream) {
@@ -918,8 +1116,8 @@ extern "C" int phb_pressure_matrix(const phb_domain *dom, const void *Adiag, voi
 		PHB_DISPATCH(dom, (kLaplaceMatrix<S, D, false, true><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)Adiag, (S *)P, P_lo)));
 		return checkLaunch("kLaplaceMatrix<non-orthogonal>");
 	}
-	PHB_DISPATCH(dom, (kLaplaceMatrix<S, D, false><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)Adiag, (S *)P, P_lo)));
-	return checkLaunch("kLaplaceMatrix");
+	PHB_DISPATCH(dom, (kPressureMatrix<S, D><<<PHB_RESIDENT(dom, (kPressureMatrix<S, D>))>>>(Dom<S, D>(*dom), (const S *)Adiag, (S *)P, P_lo)));
+	return checkLaunch("kPressureMatrix");
 }
 extern "C" int phb_epot_matrix(const phb_domain *dom, void *E, float *E_lo, phb_stream stream) {
 	if (!dom || !E) return setError(PHB_ERR_ARG, "phb_epot_matrix: null argument");
@@ -933,29 +1131,29 @@ extern "C" int phb_pressure_rhs(const phb_domain *dom, const void *C, const void
 		return setError(PHB_ERR_ARG, "phb_pressure_rhs: bad argument");
 	if (dom->ntiles == 0) return PHB_OK;
 	if (dom->scheme != 0)
-		PHB_DISPATCH(dom, (kPressureRhs<S, D, true><<<PHB_TILES(dom)>>>(quadView<S, D>(dom, {C, Adiag, u, ustar, src, hbya}),
+		PHB_DISPATCH(dom, (kPressureRhs<S, D><<<PHB_TILES(dom)>>>(quadView<S, D>(dom, {C, Adiag, u, ustar, src, hbya}),
 			(const S *)C, (const S *)Adiag, (const S *)u, (const S *)ustar, (const S *)src, src_mode, (S *)hbya)));
 	else
-		PHB_DISPATCH(dom, (kPressureRhs<S, D, false><<<PHB_TILES(dom)>>>(quadView<S, D>(dom, {C, Adiag, u, ustar, src, hbya}),
-			(const S *)C, (const S *)Adiag, (const S *)u, (const S *)ustar, (const S *)src, src_mode, (S *)hbya)));
+		PHB_DISPATCH(dom, (kPressureRhsCentral<S, D><<<PHB_RESIDENT(dom, (kPressureRhsCentral<S, D>))>>>(Dom<S, D>(*dom), (const S *)C, (const S *)Adiag, (const S *)u,
+			(const S *)ustar, (const S *)src, src_mode, (S *)hbya)));
 	return checkLaunch("kPressureRhs");
 }
 extern "C" int phb_divergence(const phb_domain *dom, const void *field, void *div, phb_stream stream) {
 	if (!dom || !field || !div) return setError(PHB_ERR_ARG, "phb_divergence: null argument");
 	if (dom->ntiles == 0) return PHB_OK;
-	PHB_DISPATCH(dom, kDivergence<S, D><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)field, (S *)div));
+	PHB_DISPATCH(dom, kDivergence<S, D><<<PHB_RESIDENT(dom, (kDivergence<S, D>))>>>(Dom<S, D>(*dom), (const S *)field, (S *)div));
 	return checkLaunch("kDivergence");
 }
 extern "C" int phb_correct_velocity(const phb_domain *dom, const void *p, const void *hbya, const void *Adiag, void *u, phb_stream stream) {
 	if (!dom || !p || !hbya || !Adiag || !u) return setError(PHB_ERR_ARG, "phb_correct_velocity: null argument");
 	if (dom->ntiles == 0) return PHB_OK;
-	PHB_DISPATCH(dom, kCorrectVelocity<S, D><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)p, (const S *)hbya, (const S *)Adiag, (S *)u));
+	PHB_DISPATCH(dom, kCorrectVelocity<S, D><<<PHB_RESIDENT(dom, (kCorrectVelocity<S, D>))>>>(Dom<S, D>(*dom), (const S *)p, (const S *)hbya, (const S *)Adiag, (S *)u));
 	return checkLaunch("kCorrectVelocity");
 }
 extern "C" int phb_uxb_epot_rhs(const phb_domain *dom, const void *u, const double *e_b, void *uxb, void *rhs, phb_stream stream) {
 	if (!dom || !u || !e_b || !uxb || !rhs) return setError(PHB_ERR_ARG, "phb_uxb_epot_rhs: null argument");
 	if (dom->ntiles == 0) return PHB_OK;
-	PHB_DISPATCH(dom, kUxbEpotRhs<S, D><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)u, e_b, (S *)uxb, (S *)rhs));
+	PHB_DISPATCH(dom, kUxbEpotRhs<S, D><<<PHB_RESIDENT(dom, (kUxbEpotRhs<S, D>))>>>(Dom<S, D>(*dom), (const S *)u, e_b, (S *)uxb, (S *)rhs));
 	return checkLaunch("kUxbEpotRhs");
 }
 extern "C" int phb_current_lorentz(const phb_domain *dom, const void *phi, const void *uxb, const double *e_b,
@@ -969,7 +1167,7 @@ extern "C" int phb_current_lorentz(const phb_domain *dom, const void *phi, const
 extern "C" int phb_epot_rhs(const phb_domain *dom, const void *field, void *rhs, phb_stream stream) {
 	if (!dom || !field || !rhs) return setError(PHB_ERR_ARG, "phb_epot_rhs: null argument");
 	if (dom->ntiles == 0) return PHB_OK;
-	PHB_DISPATCH(dom, kEpotRhs<S, D><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)field, (S *)rhs));
+	PHB_DISPATCH(dom, kEpotRhs<S, D><<<PHB_RESIDENT(dom, (kEpotRhs<S, D>))>>>(Dom<S, D>(*dom), (const S *)field, (S *)rhs));
 	return checkLaunch("kEpotRhs");
 }
 extern "C" int phb_nonortho_rhs(const phb_domain *dom, int kind, const void *field, const phb_scalar *sc, const void *Adiag,
