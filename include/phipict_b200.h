@@ -287,8 +287,8 @@ typedef struct phb_solve {
 	void *state;          /* >= phb_solve_state_bytes() bytes */
 	const phb_amg *amg;   /* optional (CG, float32, nrhs 1): precondition with one V-cycle of
 	                         this hierarchy (set up for A); its level-0 x holds z */
-	int32_t ctas_per_sm;  /* persistent kernels (use_graph 2, 3): resident CTAs per SM to launch, at
-	                         most what fits; 0: as many as fit (the grid never exceeds the tile count) */
+	int32_t ctas_per_sm;  /* persistent kernels (use_graph 2, 3): worker groups (256 threads) per SM to
+	                         launch, at most what fits; 0: as many as fit (never more than tiles) */
 	int32_t pad;
 } phb_solve;
 

@@ -19,16 +19,17 @@
 // are formed before its loads, and the loads are issued without a branch between them: a face
 // resolved by a branch of its own costs its own round trip to L2, which made most of an iteration
 // of the form before this one. Microseconds per iteration, before and after (B200):
-//   3 blocks 64x48x48 (442,368 cells, rows of four)          67 -> 44
-//   2 blocks 37x45x41 (136,530 cells, odd rows)               72 -> 41
-//   128^3 (2.1 M cells)                                      213 -> 104
-//   64 2D instances of 32^2 to 256^2 (1.2 M cells)           170 -> 91
+//   3 blocks 64x48x48 (442,368 cells, rows of four)          67 -> 42
+//   2 blocks 37x45x41 (136,530 cells, odd rows)               72 -> 39
+//   128^3 (2.1 M cells)                                      213 -> 102
+//   64 2D instances of 32^2 to 256^2 (1.2 M cells)           170 -> 77
 //   6 3D instances of 32^3 to 112^3 (3.6 M cells, odd rows)  430 -> 247
 #include "phb_krylov.cuh"
 
 namespace phb {
 
-constexpr int PCG_ITEMS = 8; // work items per phase that a CTA keeps in shared memory
+constexpr int PCG_ITEMS = 8; // work items per phase that a group keeps in shared memory
+constexpr int PCG_GROUPS = 3; // 768 threads of 80 registers
 // Four fine cells per lane in the restriction from this many fine cells on (below, two: the
 // coarse levels have too few rows to fill the chip)
 constexpr int64_t PCG_WIDE_MIN = 1 << 17;
@@ -138,7 +139,8 @@ __device__ __forceinline__ double pcgRestrictItem(const BlockTab &B, const Block
 		const float *__restrict__ A, const PcgFine<UPD> f, float *__restrict__ t, float *__restrict__ bc,
 		float *__restrict__ rOut, float *__restrict__ x, const float *__restrict__ p, float *xbest) {
 	constexpr int R = PcgRows<D>::R, H = V / 2;
-	const int grp = int(threadIdx.x) / R, rr = int(threadIdx.x) & (R - 1);
+	const int lt = int(threadIdx.x) & (PHB_TILE - 1);
+	const int grp = lt / R, rr = lt & (R - 1);
 	const int fnx = B.nx, fny = B.ny, fnz = B.nz;
 	const int cnx = CB.nx, cny = CB.ny;
 	const bool kx = cnx < fnx, ky = cny < fny, kz = D > 2 && CB.nz < fnz;
@@ -439,8 +441,9 @@ __device__ __forceinline__ void pcgDense(const AmgView<D> &mg, const SysState *s
 	const float *b = mg.b[L];
 	float *x = mg.x[L];
 	const int rows = cd.ninst * cn;
-	const int nwarps = int(gridDim.x) * NWARPS;
-	for (int row = int(blockIdx.x) * NWARPS + (threadIdx.x >> 5); row < rows; row += nwarps) {
+	// rows dealt out over the CTAs first
+	const int nwarps = int(gridDim.x) * int(blockDim.x >> 5);
+	for (int row = int(blockIdx.x) + int(gridDim.x) * int(threadIdx.x >> 5); row < rows; row += nwarps) {
 		const int inst = row / cn, r = row - inst * cn;
 		if (sst[inst].done != RUNNING) continue;
 		const int off = __ldg(cd.insts + inst * PHB_IREC + I_CELLOFF);
@@ -459,15 +462,17 @@ template <int N>
 using Count = std::integral_constant<int, N>;
 
 template <int D>
-__global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgArgs<D> a) {
+__global__ void __launch_bounds__(PHB_TILE *PCG_GROUPS, 1) kPcg(const __grid_constant__ PcgArgs<D> a) {
 	extern __shared__ __align__(16) SysState sst[];
-	__shared__ int2 sItem[(2 * AMG_MAX_LEVELS) * PCG_ITEMS]; // slot 2l: restriction of level l, 2l+1: its prolongation
+	__shared__ int2 sItems[PCG_GROUPS][(2 * AMG_MAX_LEVELS) * PCG_ITEMS]; // slot 2l: restriction of level l, 2l+1: its prolongation
 	__shared__ unsigned int sAl;
-	__shared__ double ws[TILE_SUMS * 2 * NWARPS];
+	__shared__ double sums_[PCG_GROUPS][TILE_SUMS * 2 * NWARPS];
+	const Worker wk;
+	int2 *sItem = sItems[wk.id];
+	double *ws = sums_[wk.id];
 	const int ninst = a.dom.ninst;
 	const int nblk = a.dom.nblocks;
 	const int T = a.mg.nlevels - 1;
-	const unsigned int grid = gridDim.x;
 	BlockTab *sBlk = reinterpret_cast<BlockTab *>(sst + ninst);
 	if (threadIdx.x == 0) sAl = a.vec;
 	for (int s = threadIdx.x; s < ninst; s += blockDim.x) sst[s] = a.st[s];
@@ -492,9 +497,9 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 		const int tile = it / per;
 		return make_int2(__ldg(tiles + 2 * tile), __ldg(tiles + 2 * tile + 1) + (it - tile * per) * cells);
 	};
-	for (int i = threadIdx.x; i < 2 * T * PCG_ITEMS; i += blockDim.x) {
+	for (int i = wk.lt; i < 2 * T * PCG_ITEMS; i += PHB_TILE) {
 		const int slot = i / PCG_ITEMS, l = slot >> 1;
-		const int it = int(blockIdx.x + (i % PCG_ITEMS) * grid);
+		const int it = wk.first + (i % PCG_ITEMS) * wk.step;
 		int2 w = make_int2(0, 0);
 		if (slot & 1) {
 			const int per = l ? CPT : per0;
@@ -510,7 +515,7 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 	// visit this CTA's items of a slot: f(item, block, first cell)
 	auto visit = [&](int slot, const int32_t *tiles, int n, int per, int cells, auto f) {
 		int k = 0;
-		for (int it = blockIdx.x; it < n; it += grid, ++k) {
+		for (int it = wk.first; it < n; it += wk.step, ++k) {
 			const int2 w = k < PCG_ITEMS ? sItem[slot * PCG_ITEMS + k] : decode(tiles, it, per, cells);
 			f(it, w.x, w.y);
 		}
@@ -518,7 +523,7 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 	// the same with sums over every item into the phase's partials: f(block, first cell, values)
 	auto visitSums = [&](auto count, int slot, const int32_t *tiles, int n, int per, int cells, auto f) {
 		constexpr int NV = decltype(count)::value;
-		TileSums<NV> sums{reinterpret_cast<double (*)[NV][NWARPS]>(ws), pp, 0};
+		TileSums<NV> sums{wk, reinterpret_cast<double (*)[NV][NWARPS]>(ws), pp, 0};
 		visit(slot, tiles, n, per, cells, [&](int, int b, int first) {
 			double acc[NV];
 #pragma unroll
@@ -544,7 +549,7 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 		return make_int2(__ldg(in + I_TILESTART) * perA, __ldg(in + I_TILECOUNT) * perA);
 	};
 	auto quad = [&](const BlockTab &B, int l0, auto f) {
-		const int l = l0 + 4 * int(threadIdx.x);
+		const int l = l0 + 4 * wk.lt;
 		if (l >= B.cells()) return;
 		const int row = l / B.nx, z = D > 2 ? row / B.ny : 0;
 		f(B.off + l, l - row * B.nx, row - z * B.ny, z);
@@ -552,7 +557,7 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 	// cells 256 apart (loads of a warp stay contiguous whatever the row length), two at a time
 	auto cells = [&](const BlockTab &B, int l0, auto f) {
 		const int end = min(B.cells(), l0 + cells0);
-		for (int l = l0 + int(threadIdx.x); l < end; l += 2 * PHB_TILE) {
+		for (int l = l0 + wk.lt; l < end; l += 2 * PHB_TILE) {
 			int g[2], x[2], y[2], z[2];
 			const int n = l + PHB_TILE < end ? 2 : 1;
 #pragma unroll
@@ -675,7 +680,7 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 			visit(2 * l + 1, a.mg.lv[l].tiles, a.mg.lv[l].ntiles * CPT, CPT, PHB_TILE, [&](int, int b, int first) {
 				const BlockTab &B = blk[b];
 				if (sst[B.inst].done != RUNNING) return;
-				const int c = first + int(threadIdx.x);
+				const int c = first + wk.lt;
 				if (c >= B.cells()) return;
 				const int row = c / B.nx, z = D > 2 ? row / B.ny : 0;
 				const int g = B.off + c;
@@ -770,7 +775,7 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPcg(const __grid_constant__ PcgA
 			const SysState &s = sst[B.inst];
 			if (!((s.done == MAXIT || s.done == RISING) && s.bestIt >= 0 && s.best < s.crit)) return;
 			const int end = min(B.cells(), l0 + cells0);
-			for (int l = l0 + int(threadIdx.x); l < end; l += PHB_TILE) a.x[B.off + l] = a.xbest[B.off + l];
+			for (int l = l0 + wk.lt; l < end; l += PHB_TILE) a.x[B.off + l] = a.xbest[B.off + l];
 		});
 	}
 	if (blockIdx.x == 0) {
@@ -827,15 +832,14 @@ int launchPcg(const phb_domain *dom, const phb_solve *sv, cudaStream_t s, bool s
 	a.quarter = dom->ntiles < PCG_QUARTER_TILES;
 	auto kern = kPcg<D>;
 	if (smem > 32 * 1024) PHB_CUDA(allowSmem((const void *)kern));
-	int perSM = 0;
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, PHB_TILE, smem) != cudaSuccess || perSM < 1) perSM = 1;
-	if (sv->ctas_per_sm > 0) perSM = std::min(perSM, sv->ctas_per_sm);
+	int groups = 1, ctas = 1;
+	persistentGrid(dom->ntiles * (a.quarter ? CPT : 1), PCG_GROUPS, sv->ctas_per_sm, groups, ctas);
 	cudaLaunchConfig_t cfg = {};
 	cudaLaunchAttribute attr[1];
 	attr[0].id = cudaLaunchAttributeCooperative;
 	attr[0].val.cooperative = 1;
-	cfg.gridDim = dim3(std::max(1, std::min(dom->ntiles * (a.quarter ? CPT : 1), perSM * numSMs())));
-	cfg.blockDim = dim3(PHB_TILE);
+	cfg.gridDim = dim3(ctas);
+	cfg.blockDim = dim3(PHB_TILE * groups);
 	cfg.dynamicSmemBytes = smem;
 	cfg.stream = s;
 	cfg.attrs = attr;

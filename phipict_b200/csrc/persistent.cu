@@ -10,9 +10,9 @@
 // over a warp for every row length, and the inner products are formed through shared memory in
 // the order of four consecutive cells per thread: the same bits as the per-phase kernels.
 // Measured (B200, microseconds per iteration, before -> after): CG float64 on 442,368 cells 16.6 ->
-// 15.4 and on 3.3 M cells 99 -> 91; BiCGStab float32 with three right-hand sides inside a
-// refinement on 442,368 cells 77 -> 65, on 136,530 cells (odd rows) 86 -> 69, on 2.1 M 286 -> 223,
-// with two on 64 2D instances (1.2 M) 180 -> 120.
+// 14.9 and on 3.3 M cells 99 -> 88; BiCGStab float32 with three right-hand sides inside a
+// refinement on 442,368 cells 77 -> 60, on 136,530 cells (odd rows) 86 -> 71, on 2.1 M 286 -> 211,
+// with two on 64 2D instances (1.2 M) 180 -> 100.
 #include "phb_krylov.cuh"
 
 namespace phb {
@@ -24,15 +24,16 @@ template <typename T, int D, int K>
 struct TileCtx {
 	const Dom<double, D> &dom;
 	const BlockTab *blk;
-	const int2 *items;
-	T *stage; // two tiles of values for the inner products of unaligned rows
+	Worker wk;
+	const int2 *items; // of the group
+	T *stage; // of the group: a tile of values for the inner products of unaligned rows
 	bool vec; // operands on 16-byte boundaries
 
 	// f(block, first cell) for every tile of this CTA
 	template <typename F>
 	__device__ __forceinline__ void tiles(F f) const {
 		int k = 0;
-		for (int t = blockIdx.x; t < dom.ntiles; t += gridDim.x, ++k) {
+		for (int t = wk.first; t < dom.ntiles; t += wk.step, ++k) {
 			const int2 w = k < TILE_ITEMS ? items[k] : make_int2(__ldg(dom.tiles + 2 * t), __ldg(dom.tiles + 2 * t + 1));
 			f(blk[w.x], w.y);
 		}
@@ -40,7 +41,7 @@ struct TileCtx {
 	// the same with sums over every tile into dst: f(block, first cell, values)
 	template <int NV, typename F>
 	__device__ __forceinline__ void tileSums(double *dst, double *ws, F f) const {
-		TileSums<NV> sums{reinterpret_cast<double (*)[NV][NWARPS]>(ws), dst, 0};
+		TileSums<NV> sums{wk, reinterpret_cast<double (*)[NV][NWARPS]>(ws), dst, 0};
 		tiles([&](const BlockTab &B, int l0) {
 			double acc[NV];
 #pragma unroll
@@ -132,7 +133,7 @@ __device__ __forceinline__ void tilePhase(const TileCtx<T, D, K> &cx, const Bloc
 		y = row - z * B.ny;
 	};
 	if (cx.rows4(B)) {
-		const int l = l0 + 4 * int(threadIdx.x);
+		const int l = l0 + 4 * cx.wk.lt;
 		if (l >= nc) return;
 		int x, y, z;
 		where(l, x, y, z);
@@ -151,40 +152,41 @@ __device__ __forceinline__ void tilePhase(const TileCtx<T, D, K> &cx, const Bloc
 	T yv[CPT][K], fv[CPT][K];
 #pragma unroll
 	for (int j = 0; j < CPT; ++j) {
-		const int l = l0 + int(threadIdx.x) + j * PHB_TILE;
+		const int l = l0 + cx.wk.lt + j * PHB_TILE;
 		const int lc = l < nc ? l : l0; // past the end: the tile's first cell, not used
 		int x, y, z;
 		where(lc, x, y, z);
 		cellApply<T, D, K>(B, B.off + lc, x, y, z, N, A, act, fld, yv[j], fv[j]);
 	}
-	T *ys = cx.stage, *fs = cx.stage + PHB_TILE_CELLS;
-	const int q0 = 4 * int(threadIdx.x);
+	const int q0 = 4 * cx.wk.lt;
 	const int n = max(0, min(4, nc - l0 - q0));
 #pragma unroll
 	for (int k = 0; k < K; ++k) {
 		if (!act[k]) continue;
 		const int64_t d = TileCtx<T, D, K>::base(B, k) + B.off;
-		__syncthreads();
+		T y4[4], f4[4];
+		// y, then f, from the thread that has the cell to the thread that sums it
+		auto pass = [&](auto value, T(&v4)[4]) {
+			cx.wk.sync();
+#pragma unroll
+			for (int j = 0; j < CPT; ++j) cx.stage[cx.wk.lt + j * PHB_TILE] = value(j);
+			cx.wk.sync();
+#pragma unroll
+			for (int i = 0; i < 4; ++i) v4[i] = i < n ? cx.stage[q0 + i] : T(0);
+		};
 #pragma unroll
 		for (int j = 0; j < CPT; ++j) {
-			const int c = int(threadIdx.x) + j * PHB_TILE;
+			const int c = cx.wk.lt + j * PHB_TILE;
 			if (l0 + c < nc) {
 				const T y1[4] = {yv[j][k], 0, 0, 0}, f1[4] = {fv[j][k], 0, 0, 0};
 				emit(k, d + l0 + c, 1, y1, f1);
-				ys[c] = yv[j][k];
-				fs[c] = fv[j][k];
 			}
 		}
-		__syncthreads();
-		T y4[4], f4[4];
-#pragma unroll
-		for (int i = 0; i < 4; ++i) {
-			y4[i] = i < n ? ys[q0 + i] : T(0);
-			f4[i] = i < n ? fs[q0 + i] : T(0);
-		}
+		pass([&](int j) { return yv[j][k]; }, y4);
+		pass([&](int j) { return fv[j][k]; }, f4);
 		dots(k, d + l0 + q0, n, y4, f4, acc);
 	}
-	__syncthreads();
+	cx.wk.sync();
 }
 
 // values of a row of four (n = 4 with vec) or of the first n of four cells
@@ -223,29 +225,41 @@ __device__ __forceinline__ void residualTile(const TileCtx<T, D, K> &cx, const B
 // Shared prologue of the persistent kernels: states, block tables, tile list.
 template <typename T, int D, int K>
 __device__ __forceinline__ TileCtx<T, D, K> tileContext(const Dom<double, D> &dom, const BlockTab *blocks, SysState *sst, const SysState *st,
-		int2 *items, T *stage) {
+		int2 (*items)[TILE_ITEMS], T (*stage)[PHB_TILE_CELLS]) {
+	const Worker wk;
 	const int nsys = dom.ninst * K;
 	BlockTab *sBlk = reinterpret_cast<BlockTab *>(sst + nsys);
 	for (int s = threadIdx.x; s < nsys; s += blockDim.x) sst[s] = st[s];
 	if (!blocks)
 		for (int b = threadIdx.x; b < dom.nblocks; b += blockDim.x) buildBlockTab<D>(dom.blocks, b, sBlk[b]);
-	if (threadIdx.x < TILE_ITEMS) {
-		const int t = int(blockIdx.x + threadIdx.x * gridDim.x);
-		items[threadIdx.x] = t < dom.ntiles ? make_int2(__ldg(dom.tiles + 2 * t), __ldg(dom.tiles + 2 * t + 1)) : make_int2(0, 0);
+	if (wk.lt < TILE_ITEMS) {
+		const int t = wk.first + wk.lt * wk.step;
+		items[wk.id][wk.lt] = t < dom.ntiles ? make_int2(__ldg(dom.tiles + 2 * t), __ldg(dom.tiles + 2 * t + 1)) : make_int2(0, 0);
 	}
 	__syncthreads();
-	return TileCtx<T, D, K>{dom, blocks ? blocks : sBlk, items, stage, dom.vec4 != 0};
+	return TileCtx<T, D, K>{dom, blocks ? blocks : sBlk, wk, items[wk.id], stage[wk.id], dom.vec4 != 0};
 }
+
+// Worker groups per CTA: float32 with one right-hand side is bound by HBM on large grids and is
+// faster with more warps in flight (four groups of 64 registers a thread); several right-hand sides
+// and float64 need more registers.
+template <typename T, int D, int K>
+constexpr int cgGroups() {
+	return (std::is_same<T, float>::value && K == 1) ? 4 : (K == 1 ? 3 : 2);
+}
+constexpr int BICG_GROUPS = 2;
 
 template <typename T, int D, int K, bool STOPSTART>
 __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, const BlockTab *blocks, const T *__restrict__ A, const T *__restrict__ b,
 		T *__restrict__ x, T *__restrict__ r, T *__restrict__ p0, T *__restrict__ p1, T *__restrict__ q, T *__restrict__ xbest,
 		SysState *st, double *partial, Control *ctrl, const phb_tolerance &tol, int returnBest, int maxit) {
 	extern __shared__ __align__(16) SysState sst[];
-	__shared__ int2 items[TILE_ITEMS];
-	__shared__ __align__(16) T stage[2 * PHB_TILE_CELLS];
-	__shared__ double ws[TILE_SUMS * 2 * K * NWARPS];
+	constexpr int G = cgGroups<T, D, K>();
+	__shared__ int2 items[G][TILE_ITEMS];
+	__shared__ __align__(16) T stage[G][PHB_TILE_CELLS];
+	__shared__ double sums[G][TILE_SUMS * 2 * K * NWARPS];
 	const TileCtx<T, D, K> cx = tileContext<T, D, K>(dom, blocks, sst, st, items, stage);
+	double *ws = sums[cx.wk.id];
 	const int64_t N = dom.ncells;
 	auto range = [&](int inst) {
 		const int32_t *in = dom.insts + inst * PHB_IREC;
@@ -300,7 +314,7 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 		// x += alpha p', r -= alpha q, (r, r)
 		pp = partial + (size_t)(ph++ & 1) * half;
 		cx.template tileSums<K>(pp, ws, [&](const BlockTab &B, int l0, double (&acc)[K]) {
-			const int l = l0 + 4 * int(threadIdx.x);
+			const int l = l0 + 4 * cx.wk.lt;
 			const int n = max(0, min(4, B.cells() - l));
 			const bool al = cx.rows4(B) && n == 4;
 #pragma unroll
@@ -358,7 +372,7 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 				const SysState &s = sst[B.inst * K + k];
 				if (!((s.done == MAXIT || s.done == RISING) && s.bestIt >= 0 && s.best < s.crit)) continue;
 				const int64_t d = B.off + cx.base(B, k);
-				for (int l = l0 + int(threadIdx.x); l < end; l += PHB_TILE) x[d + l] = xbest[d + l];
+				for (int l = l0 + cx.wk.lt; l < end; l += PHB_TILE) x[d + l] = xbest[d + l];
 			}
 		});
 	}
@@ -368,30 +382,24 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 	}
 }
 
-// Resident CTAs per SM that the register budget must allow: float32 with one right-hand side is
-// bound by HBM on large grids and is faster with more warps in flight; several right-hand sides and
-// float64 need more registers per thread.
-template <typename T, int D, int K>
-constexpr int cgMinBlocks() {
-	return (std::is_same<T, float>::value && K == 1) ? 4 : (K == 1 ? 3 : 2);
-}
-
 template <typename T, int D, int K, bool STOPSTART>
-__global__ void __launch_bounds__(PHB_TILE, (cgMinBlocks<T, D, K>())) kCgPersistent(Dom<double, D> dom, const BlockTab *blocks, const T *__restrict__ A,
+__global__ void __launch_bounds__(PHB_TILE * cgGroups<T, D, K>(), 1) kCgPersistent(Dom<double, D> dom, const BlockTab *blocks, const T *__restrict__ A,
 		const T *__restrict__ b, T *__restrict__ x, T *__restrict__ r, T *__restrict__ p0, T *__restrict__ p1, T *__restrict__ q,
 		T *__restrict__ xbest, SysState *st, double *partial, Control *ctrl, phb_tolerance tol, int returnBest, int maxit) {
 	cgPersistentBody<T, D, K, STOPSTART>(dom, blocks, A, b, x, r, p0, p1, q, xbest, st, partial, ctrl, tol, returnBest, maxit);
 }
 
 template <typename T, int D, int K>
-__global__ void __launch_bounds__(PHB_TILE, 2) kBicgPersistent(Dom<double, D> dom, const BlockTab *blocks, const T *__restrict__ A, const T *__restrict__ b,
+__global__ void __launch_bounds__(PHB_TILE *BICG_GROUPS, 1) kBicgPersistent(Dom<double, D> dom, const BlockTab *blocks, const T *__restrict__ A, const T *__restrict__ b,
 		T *__restrict__ x, T *__restrict__ r, T *__restrict__ r0, T *__restrict__ p0, T *__restrict__ p1, T *__restrict__ v0,
 		T *__restrict__ v1, T *__restrict__ t, SysState *st, double *partial, Control *ctrl, phb_tolerance tol, int maxit) {
 	extern __shared__ __align__(16) SysState sst[];
-	__shared__ int2 items[TILE_ITEMS];
-	__shared__ __align__(16) T stage[2 * PHB_TILE_CELLS];
-	__shared__ double ws[TILE_SUMS * 3 * K * NWARPS];
+	constexpr int G = BICG_GROUPS;
+	__shared__ int2 items[G][TILE_ITEMS];
+	__shared__ __align__(16) T stage[G][PHB_TILE_CELLS];
+	__shared__ double sums[G][TILE_SUMS * 3 * K * NWARPS];
 	const TileCtx<T, D, K> cx = tileContext<T, D, K>(dom, blocks, sst, st, items, stage);
+	double *ws = sums[cx.wk.id];
 	const int64_t N = dom.ncells;
 	auto range = [&](int inst) {
 		const int32_t *in = dom.insts + inst * PHB_IREC;
@@ -485,7 +493,7 @@ __global__ void __launch_bounds__(PHB_TILE, 2) kBicgPersistent(Dom<double, D> do
 		// x += alpha p + omega s, r = s - omega t, (r0, r), (r, r)
 		pp = partial + (size_t)(ph++ & 1) * half;
 		cx.template tileSums<2 * K>(pp, ws, [&](const BlockTab &B, int l0, double (&acc)[2 * K]) {
-			const int l = l0 + 4 * int(threadIdx.x);
+			const int l = l0 + 4 * cx.wk.lt;
 			const int n = max(0, min(4, B.cells() - l));
 			const bool al = cx.rows4(B) && n == 4;
 #pragma unroll
@@ -599,23 +607,24 @@ int launchPersistent(const phb_domain *dom, const phb_solve *sv, cudaStream_t s,
 	cudaLaunchAttribute attr[1];
 	attr[0].id = cudaLaunchAttributeCooperative;
 	attr[0].val.cooperative = 1;
-	cfg.blockDim = dim3(PHB_TILE);
 	cfg.dynamicSmemBytes = smem;
 	cfg.stream = s;
 	cfg.attrs = attr;
 	cfg.numAttrs = 1;
-	auto grid = [&](const void *kern) -> int {
-		if (smem > 16 * 1024) (void)allowSmem(kern);
-		int perSM = 0;
-		if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, PHB_TILE, smem) != cudaSuccess || perSM < 1) perSM = 1;
-		if (sv->ctas_per_sm > 0) perSM = std::min(perSM, sv->ctas_per_sm); // a tuned, smaller grid
-		return std::max(1, std::min(dom->ntiles, perSM * numSMs()));
+	auto configure = [&](const void *kern, int most) -> int {
+		if (smem > 8 * 1024) PHB_CUDA(allowSmem(kern));
+		int groups = 1, ctas = 1;
+		persistentGrid(dom->ntiles, most, sv->ctas_per_sm, groups, ctas);
+		cfg.gridDim = dim3(ctas);
+		cfg.blockDim = dim3(PHB_TILE * groups);
+		return PHB_OK;
 	};
 	if (sv->kind == 0) {
 		T *r = (T *)(w + L.off[0]), *q = (T *)(w + L.off[1]), *p0 = (T *)(w + L.off[2]), *p1 = (T *)(w + L.off[3]);
 		T *xbest = sv->return_best ? (T *)(w + L.off[4]) : nullptr;
 		auto launch = [&](auto kern) -> int {
-			cfg.gridDim = dim3(grid((const void *)kern));
+			const int rc2 = configure((const void *)kern, cgGroups<T, D, K>());
+			if (rc2) return rc2;
 			PHB_CUDA(cudaLaunchKernelEx(&cfg, kern, dm, tabs, A, b, x, r, p0, p1, q, xbest, st, partial, ctrl, sv->tol, sv->return_best, maxit));
 			return PHB_OK;
 		};
@@ -624,7 +633,8 @@ int launchPersistent(const phb_domain *dom, const phb_solve *sv, cudaStream_t s,
 	T *r = (T *)(w + L.off[0]), *r0 = (T *)(w + L.off[1]), *p0 = (T *)(w + L.off[2]), *p1 = (T *)(w + L.off[3]);
 	T *v0 = (T *)(w + L.off[4]), *v1 = (T *)(w + L.off[5]), *t = (T *)(w + L.off[6]);
 	auto kern = kBicgPersistent<T, D, K>;
-	cfg.gridDim = dim3(grid((const void *)kern));
+	const int rc2 = configure((const void *)kern, BICG_GROUPS);
+	if (rc2) return rc2;
 	PHB_CUDA(cudaLaunchKernelEx(&cfg, kern, dm, tabs, A, b, x, r, r0, p0, p1, v0, v1, t, st, partial, ctrl, sv->tol, maxit));
 	return PHB_OK;
 }

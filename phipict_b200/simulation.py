@@ -17,7 +17,7 @@ Extensions (keyword arguments phiPICT does not have):
   ``check_solves``: read the solver outcomes at the end of every step (default True).
       With False the step never synchronises; failures surface through
       :meth:`solve_report`.
-  ``autotune_solvers``: measure and pick the CTAs per SM of each solve (SolverTuner).
+  ``autotune_solvers``: measure and pick the worker groups per SM of each solve (SolverTuner).
   ``extrapolate_guesses``: start the pressure and potential solves from a polynomial
       extrapolation of their last results (a degree m >= 1, True: 1, or "adaptive") or from
       the Galerkin projection onto the span of the last L results ("projection[:L]", 12).

@@ -203,13 +203,13 @@ class RefinedSolver:
 
 
 class SolverTuner:
-    """Per-solve tuning of the persistent Krylov kernels' grid (resident CTAs per SM), by
+    """Per-solve tuning of the persistent Krylov kernels' grid (worker groups per SM), by
     measurement: the first ``trials`` x len(CANDIDATES) solves of each tag (``velocity``,
     ``pressure0``, ``epot``, ...) cycle through the candidates, each timed with CUDA events and
     divided by its iterations (the slowest system's; inner iterations under refinement); from
-    then on the tag runs with the candidate of the lowest median time per iteration. 0 is the
-    occupancy maximum (one CTA per tile where the grid allows), smaller values launch fewer,
-    fuller CTAs. A choice changes the launch only, never the arithmetic: the results of every
+    then on the tag runs with the candidate of the lowest median time per iteration. 0 is as many
+    groups of 256 threads as fit (one per tile where the grid allows), smaller values launch fewer
+    with more tiles each. A choice changes the launch only, never the arithmetic: the results of every
     candidate are the same bits."""
 
     CANDIDATES = (0, 2, 1)
