@@ -119,6 +119,60 @@ def test_projection_gram_matches_torch(cuda, m, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m", [2, 3, 4, 8, 9, 15])
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 100003])
+def test_projection_gram_at_the_edges_of_its_tiles(cuda, m, n):
+    """Row counts around the 3 x 3 register tiles, lengths around the chunk of 128. Each entry is
+    a sum of n products of standard normals, in any order: error below n eps times sum |v y|."""
+    from phipict_b200 import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(m)
+    stride = n + 5
+    V = torch.randn(m, stride, dtype=torch.float64, device="cuda", generator=g)
+    Y = torch.randn(m, stride, dtype=torch.float64, device="cuda", generator=g)
+    b = torch.randn(n, dtype=torch.float64, device="cuda", generator=g)
+    G = torch.full((m, m), float("nan"), dtype=torch.float64, device="cuda")
+    c = torch.full((m,), float("nan"), dtype=torch.float64, device="cuda")
+    _lib.call("phb_projection_gram", V.data_ptr(), Y.data_ptr(), b.data_ptr(), m, n, stride, G.data_ptr(), c.data_ptr(),
+              _lib.stream_ptr(V.device))
+    v, y = V[:, :n], Y[:, :n]
+    eps = n * 2.0 ** -52
+    assert ((G - v @ y.T).abs() <= eps * (v.abs() @ y.abs().T)).all()
+    assert ((c - v @ b).abs() <= eps * (v.abs() @ b.abs())).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", ["odd_3d", "thin_3d", "rotated_2d", "batch"])
+def test_stencil_apply_on_other_shapes(cuda, shape):
+    """Odd rows, partial tiles, blocks one cell thick, connections that swap axes, a batch: against
+    torch's CSR product, 2 D + 1 products per row."""
+    import ctypes as ct
+
+    from cases import duct_3d, rotated_pair_2d
+    from phipict_b200 import _lib
+
+    dom = {"odd_3d": lambda: duct_3d(13, 11, 9, 3), "thin_3d": lambda: duct_3d(20, 1, 24, 1),
+           "rotated_2d": lambda: rotated_pair_2d(16), "batch": lambda: hartmann_2d(33, 31, batch=3)}[shape]()
+    seeded_state(dom, 3, scale=0.2)
+    dom.PrepareSolve()
+    sim = pb.Simulation(dom, 1e-2, non_orthogonal=False)
+    assert sim.single_step(), sim.last_error
+    N = dom.getTotalSize()
+    g = torch.Generator(device="cuda").manual_seed(6)
+    X = torch.randn(2, N + 8, dtype=torch.float64, device="cuda", generator=g)
+    Y = torch.full_like(X, float("nan"))
+    _lib.call("phb_stencil_apply", ct.byref(dom.desc()), dom._stencil("P").data_ptr(), X.data_ptr(), Y.data_ptr(), 2,
+              X.stride(0), _lib.stream_ptr(X.device))
+    M = dom.P
+    A = torch.sparse_csr_tensor(M.row.to(torch.int64), M.index.to(torch.int64), M.value, size=(N, N))
+    absA = torch.sparse_csr_tensor(M.row.to(torch.int64), M.index.to(torch.int64), M.value.abs(), size=(N, N))
+    for v in range(2):
+        ref, mag = torch.mv(A, X[v, :N].contiguous()), torch.mv(absA, X[v, :N].abs().contiguous())
+        assert ((Y[v, :N] - ref).abs() <= 8 * 2.0 ** -52 * mag).all()
+        assert torch.isnan(Y[v, N:]).all()
+
+
+@pytest.mark.gpu
 def test_projection_solve_matches_a_dense_solve(cuda):
     """phb_projection_solve against torch.linalg.solve on symmetric definite systems of both
     signs, and the coefficient 0 of a row that is linearly dependent on the others."""
