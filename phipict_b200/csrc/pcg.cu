@@ -21,9 +21,9 @@
 // of the form before this one. Microseconds per iteration, before and after (B200):
 //   3 blocks 64x48x48 (442,368 cells, rows of four)          67 -> 42
 //   2 blocks 37x45x41 (136,530 cells, odd rows)               72 -> 39
-//   128^3 (2.1 M cells)                                      213 -> 102
+//   128^3 (2.1 M cells)                                      213 -> 99
 //   64 2D instances of 32^2 to 256^2 (1.2 M cells)           170 -> 77
-//   6 3D instances of 32^3 to 112^3 (3.6 M cells, odd rows)  430 -> 247
+//   6 3D instances of 32^3 to 112^3 (3.6 M cells, odd rows)  430 -> 226
 #include "phb_krylov.cuh"
 
 namespace phb {
@@ -465,6 +465,7 @@ template <int D>
 __global__ void __launch_bounds__(PHB_TILE *PCG_GROUPS, 1) kPcg(const __grid_constant__ PcgArgs<D> a) {
 	extern __shared__ __align__(16) SysState sst[];
 	__shared__ int2 sItems[PCG_GROUPS][(2 * AMG_MAX_LEVELS) * PCG_ITEMS]; // slot 2l: restriction of level l, 2l+1: its prolongation
+	__shared__ int sCount[PCG_GROUPS][2]; // the group's items of slots 0 and 1
 	__shared__ unsigned int sAl;
 	__shared__ double sums_[PCG_GROUPS][TILE_SUMS * 2 * NWARPS];
 	const Worker wk;
@@ -509,13 +510,21 @@ __global__ void __launch_bounds__(PHB_TILE *PCG_GROUPS, 1) kPcg(const __grid_con
 		}
 		sItem[i] = w;
 	}
+	if (wk.lt < 2) sCount[wk.id][wk.lt] = wk.count(wk.lt ? a.dom.ntiles * per0 : a.mg.lv[1].ntiles * perR(0));
 	__syncthreads();
 	int ph = 0;
 	double *pp = a.partial;
-	// visit this CTA's items of a slot: f(item, block, first cell)
+	// Visit the group's items of a slot: f(item, block, first cell). The passes over the finest level
+	// alternate in direction: what the one before touched last is still in L2 (six odd ducts of 3.6 M cells 250 -> 226 us per
+	// iteration, with the reduction's wider loads).
+	bool back = false;
 	auto visit = [&](int slot, const int32_t *tiles, int n, int per, int cells, auto f) {
-		int k = 0;
-		for (int it = wk.first; it < n; it += wk.step, ++k) {
+		int k = 0, it = wk.first, dk = 1;
+		if (slot < 2) {
+			if (back) { k = sCount[wk.id][slot] - 1; it += k * wk.step; dk = -1; }
+			back = !back;
+		}
+		for (; dk < 0 ? k >= 0 : it < n; k += dk, it += dk * wk.step) {
 			const int2 w = k < PCG_ITEMS ? sItem[slot * PCG_ITEMS + k] : decode(tiles, it, per, cells);
 			f(it, w.x, w.y);
 		}
@@ -523,7 +532,7 @@ __global__ void __launch_bounds__(PHB_TILE *PCG_GROUPS, 1) kPcg(const __grid_con
 	// the same with sums over every item into the phase's partials: f(block, first cell, values)
 	auto visitSums = [&](auto count, int slot, const int32_t *tiles, int n, int per, int cells, auto f) {
 		constexpr int NV = decltype(count)::value;
-		TileSums<NV> sums{wk, reinterpret_cast<double (*)[NV][NWARPS]>(ws), pp, 0};
+		TileSums<NV> sums{wk, reinterpret_cast<double (*)[NV][NWARPS]>(ws), pp, 0, back ? sCount[wk.id][slot] - 1 : -1};
 		visit(slot, tiles, n, per, cells, [&](int, int b, int first) {
 			double acc[NV];
 #pragma unroll

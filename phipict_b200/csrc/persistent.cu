@@ -10,8 +10,8 @@
 // over a warp for every row length, and the inner products are formed through shared memory in
 // the order of four consecutive cells per thread: the same bits as the per-phase kernels.
 // Measured (B200, microseconds per iteration, before -> after): CG float64 on 442,368 cells 16.6 ->
-// 14.9 and on 3.3 M cells 99 -> 88; BiCGStab float32 with three right-hand sides inside a
-// refinement on 442,368 cells 77 -> 60, on 136,530 cells (odd rows) 86 -> 71, on 2.1 M 286 -> 211,
+// 14.3 and on 3.3 M cells 99 -> 81; BiCGStab float32 with three right-hand sides inside a
+// refinement on 442,368 cells 77 -> 60, on 136,530 cells (odd rows) 86 -> 67, on 2.1 M 286 -> 192,
 // with two on 64 2D instances (1.2 M) 180 -> 100.
 #include "phb_krylov.cuh"
 
@@ -28,20 +28,25 @@ struct TileCtx {
 	const int2 *items; // of the group
 	T *stage; // of the group: a tile of values for the inner products of unaligned rows
 	bool vec; // operands on 16-byte boundaries
+	int n;    // the group's tiles
+	// Every phase visits them in the opposite order of the phase before: what that one touched last
+	// (up to the 126 MB of L2) is read from L2, where in the same order it would just have been
+	// evicted (CG on 3.3 M float64 cells 88 -> 81 us, with the reduction's wider loads).
+	bool back;
 
-	// f(block, first cell) for every tile of this CTA
+	// f(block, first cell) for every tile of this group
 	template <typename F>
 	__device__ __forceinline__ void tiles(F f) const {
-		int k = 0;
-		for (int t = wk.first; t < dom.ntiles; t += wk.step, ++k) {
+		for (int i = 0; i < n; ++i) {
+			const int k = back ? n - 1 - i : i, t = wk.first + k * wk.step;
 			const int2 w = k < TILE_ITEMS ? items[k] : make_int2(__ldg(dom.tiles + 2 * t), __ldg(dom.tiles + 2 * t + 1));
 			f(blk[w.x], w.y);
 		}
 	}
 	// the same with sums over every tile into dst: f(block, first cell, values)
 	template <int NV, typename F>
-	__device__ __forceinline__ void tileSums(double *dst, double *ws, F f) const {
-		TileSums<NV> sums{wk, reinterpret_cast<double (*)[NV][NWARPS]>(ws), dst, 0};
+	__device__ __forceinline__ void tileSums(double *dst, double *ws, F f) {
+		TileSums<NV> sums{wk, reinterpret_cast<double (*)[NV][NWARPS]>(ws), dst, 0, back ? n - 1 : -1};
 		tiles([&](const BlockTab &B, int l0) {
 			double acc[NV];
 #pragma unroll
@@ -51,6 +56,7 @@ struct TileCtx {
 			sums.next();
 		});
 		sums.finish();
+		back = !back;
 	}
 	__device__ __forceinline__ bool rows4(const BlockTab &B) const {
 		return vec && B.rows4() && (K == 1 || ((B.instOff | B.instN) & 3) == 0);
@@ -237,7 +243,7 @@ __device__ __forceinline__ TileCtx<T, D, K> tileContext(const Dom<double, D> &do
 		items[wk.id][wk.lt] = t < dom.ntiles ? make_int2(__ldg(dom.tiles + 2 * t), __ldg(dom.tiles + 2 * t + 1)) : make_int2(0, 0);
 	}
 	__syncthreads();
-	return TileCtx<T, D, K>{dom, blocks ? blocks : sBlk, wk, items[wk.id], stage[wk.id], dom.vec4 != 0};
+	return TileCtx<T, D, K>{dom, blocks ? blocks : sBlk, wk, items[wk.id], stage[wk.id], dom.vec4 != 0, wk.count(dom.ntiles), false};
 }
 
 // Worker groups per CTA: float32 with one right-hand side is bound by HBM on large grids and is
@@ -258,7 +264,7 @@ __device__ __forceinline__ void cgPersistentBody(const Dom<double, D> &dom, cons
 	__shared__ int2 items[G][TILE_ITEMS];
 	__shared__ __align__(16) T stage[G][PHB_TILE_CELLS];
 	__shared__ double sums[G][TILE_SUMS * 2 * K * NWARPS];
-	const TileCtx<T, D, K> cx = tileContext<T, D, K>(dom, blocks, sst, st, items, stage);
+	TileCtx<T, D, K> cx = tileContext<T, D, K>(dom, blocks, sst, st, items, stage);
 	double *ws = sums[cx.wk.id];
 	const int64_t N = dom.ncells;
 	auto range = [&](int inst) {
@@ -398,7 +404,7 @@ __global__ void __launch_bounds__(PHB_TILE *BICG_GROUPS, 1) kBicgPersistent(Dom<
 	__shared__ int2 items[G][TILE_ITEMS];
 	__shared__ __align__(16) T stage[G][PHB_TILE_CELLS];
 	__shared__ double sums[G][TILE_SUMS * 3 * K * NWARPS];
-	const TileCtx<T, D, K> cx = tileContext<T, D, K>(dom, blocks, sst, st, items, stage);
+	TileCtx<T, D, K> cx = tileContext<T, D, K>(dom, blocks, sst, st, items, stage);
 	double *ws = sums[cx.wk.id];
 	const int64_t N = dom.ncells;
 	auto range = [&](int inst) {
