@@ -105,3 +105,21 @@ def test_persistent_solvers_of_a_batch(cuda, sizes):
     b = _rhs(batch, batch.numCells(), 2, 4)
     ref = _solve(batch, BICGSTAB, 2, batch._C_st, b, 1e-8, 500, 1)
     assert _same(_solve(batch, BICGSTAB, 2, batch._C_st, b, 1e-8, 500, 2), ref)
+
+
+@pytest.mark.parametrize("kind", [CG, BICGSTAB], ids=["cg", "bicgstab"])
+def test_block_tables_that_do_not_fit_shared_memory(cuda, kind):
+    """500 instances: the tables of their blocks go to global memory; still the per-phase kernels' bits."""
+    dom = hartmann_2d(9, 7)
+    dom.setBatchSize(500)
+    dom.PrepareSolve()
+    g = torch.Generator().manual_seed(2)
+    v = dom.getBlocks()[0].velocity
+    v.copy_((1.0 + 0.2 * torch.randn(v.shape, generator=g, dtype=torch.float64)).to(v.device, v.dtype))
+    _assemble(dom, 2)
+    nrhs = 1 if kind == CG else 2
+    A, tol = (dom._P_st, 1e-6) if kind == CG else (dom._C_st, 1e-8)
+    b = _rhs(dom, dom.numCells(), nrhs, 3)
+    ref = _solve(dom, kind, nrhs, A, b, tol, 1000, 1)
+    assert all(i.converged for i in ref[1])
+    assert _same(_solve(dom, kind, nrhs, A, b, tol, 1000, 2, ctas=1), ref)
