@@ -574,6 +574,10 @@ int launchPersistent(const phb_domain *dom, const phb_solve *sv, cudaStream_t s,
 	if constexpr (std::is_same<T, float>::value && K == 1) {
 		if (sv->amg && sv->kind == 0) return launchPcg<D>(dom, sv, s, stopStart, fromInner);
 	}
+	const int nsys = dom->ninst * K;
+	const size_t stBytes = (size_t)nsys * sizeof(SysState);
+	// the limit of the grid kernels' state copies, and of the mode: the same for every kernel it may pick
+	if (stBytes > 160 * 1024) return setError(PHB_ERR_RANGE, "persistent solve: too many systems for the per-CTA state copy");
 	if constexpr (K == 1) {
 		if (sv->kind == 0) {
 			bool taken = false;
@@ -593,9 +597,6 @@ int launchPersistent(const phb_domain *dom, const phb_solve *sv, cudaStream_t s,
 	const T *b = (const T *)sv->b;
 	T *x = (T *)sv->x;
 	dm.vec4 = vec4Ok(dom, {A, b, x, w});
-	const int nsys = dom->ninst * K;
-	const size_t stBytes = (size_t)nsys * sizeof(SysState);
-	if (stBytes > 160 * 1024) return setError(PHB_ERR_RANGE, "persistent solve: too many systems for the per-CTA state copy");
 	const int maxit = std::max(1, sv->maxit);
 	const int rc = launchInit(st, nsys, sv->tol, fromInner, maxit, ctrl, s);
 	if (rc) return rc;

@@ -123,3 +123,15 @@ def test_block_tables_that_do_not_fit_shared_memory(cuda, kind):
     ref = _solve(dom, kind, nrhs, A, b, tol, 1000, 1)
     assert all(i.converged for i in ref[1])
     assert _same(_solve(dom, kind, nrhs, A, b, tol, 1000, 2, ctas=1), ref)
+
+
+@pytest.mark.parametrize("kind,nrhs,instances", [(CG, 1, 1281), (CG, 2, 641), (BICGSTAB, 1, 1281), (BICGSTAB, 2, 641)])
+def test_more_systems_than_a_cta_keeps_states_of_are_refused(cuda, kind, nrhs, instances):
+    """160 KB of states, 1280 systems: the persistent mode refuses more whichever kernel would run."""
+    dom = hartmann_2d(5, 4)
+    dom.setBatchSize(instances)
+    dom.PrepareSolve()
+    b = torch.ones(dom.numCells() * nrhs, dtype=torch.float64, device=cuda)
+    A = dom._P_st if kind == CG else dom._C_st
+    with pytest.raises(RuntimeError, match="too many systems"):
+        _solve(dom, kind, nrhs, A, b, 1e-6, 10, 2)
