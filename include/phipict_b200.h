@@ -288,7 +288,9 @@ typedef struct phb_solve {
 	const phb_amg *amg;   /* optional (CG, float32, nrhs 1): precondition with one V-cycle of
 	                         this hierarchy (set up for A); its level-0 x holds z */
 	int32_t ctas_per_sm;  /* persistent kernels (use_graph 2, 3): worker groups (256 threads) per SM to
-	                         launch, at most what fits; 0: as many as fit (never more than tiles) */
+	                         launch, at most what fits; 0: as many as fit (never more than tiles), and a CG
+	                         of small instances (at most 32 tiles) may run as one cluster per instance,
+	                         which any other value rules out */
 	int32_t pad;
 } phb_solve;
 

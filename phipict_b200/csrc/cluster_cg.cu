@@ -306,8 +306,20 @@ __global__ void __launch_bounds__(PHB_TILE *CCG_SLOTS, 1) kCgCluster(const __gri
 	clusterBarrier(); // no CTA leaves while another may still read its shared memory
 }
 
+// Whether `ninst` clusters, `resident` of them at a time, beat the grid-wide kernel: its iteration takes
+// about 8 us and 0.24 us more per instance (every SM sums every system; flat from some 128 instances
+// on), a cluster's 3.7 us. Every cluster has the size that the largest instance may have, so a batch of many
+// small instances and one large one holds few at a time. Measured (microseconds per iteration of all, cluster
+// and grid): 22 instances of 2 tiles in clusters of 32 tiles, 7 at a time, 13.3 and 11.5, 16 of them
+// 10.2 and 10.3; 64 in clusters of 16 tiles, 14 at a time, 15.7 and 22.7; 301 66 and 38; 301 in clusters of 8 29 and 38.
+inline bool clustersWin(int ninst, int resident) {
+	const int64_t waves = (ninst + resident - 1) / resident;
+	return 31 * waves <= 66 + 2 * std::min(ninst, 128);
+}
+
 // Launch the cluster solve when every instance fits a cluster (the largest has at most all tiles but
-// one per other instance) and the device can hold such a cluster; *taken says whether it did.
+// one per other instance), the device can hold such a cluster and holds enough of them at a time;
+// *taken says whether it did.
 template <typename T, int D>
 int launchClusterCg(const phb_domain *dom, const phb_solve *sv, cudaStream_t s, bool stopStart, int fromInner, bool *taken) {
 	*taken = false;
@@ -329,21 +341,23 @@ int launchClusterCg(const phb_domain *dom, const phb_solve *sv, cudaStream_t s, 
 	cfg.stream = s;
 	cfg.attrs = attr;
 	cfg.numAttrs = 1;
-	// 1: such clusters fit this device, -1: they do not (asked once per device and shape)
-	static std::atomic<signed char> fits[64][CCG_SLOTS][5];
+	// such clusters that this device holds at a time, -1: none (asked once per device and shape)
+	static std::atomic<int> fits[64][CCG_SLOTS][5];
 	int dev = 0;
 	PHB_CUDA(cudaGetDevice(&dev));
 	if (dev < 0 || dev >= 64) return PHB_OK;
-	signed char ok = fits[dev][slots - 1][lg].load();
-	if (ok == 0) {
+	int resident = fits[dev][slots - 1][lg].load();
+	if (resident == 0) {
 		PHB_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CCG_SLOTS * 3 * PHB_TILE_CELLS * (int)sizeof(T)));
 		PHB_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
 		int n = 0;
-		ok = cudaOccupancyMaxActiveClusters(&n, (const void *)kern, &cfg) == cudaSuccess && n >= 1 ? 1 : -1;
-		if (ok < 0) (void)cudaGetLastError();
-		fits[dev][slots - 1][lg].store(ok);
+		cudaLaunchConfig_t full = cfg; // the device's capacity, whatever this launch's grid
+		full.gridDim = dim3(csize * numSMs());
+		resident = cudaOccupancyMaxActiveClusters(&n, (const void *)kern, &full) == cudaSuccess && n >= 1 ? n : -1;
+		if (resident < 0) (void)cudaGetLastError();
+		fits[dev][slots - 1][lg].store(resident);
 	}
-	if (ok < 0) return PHB_OK;
+	if (resident < 0 || !clustersWin(dom->ninst, resident)) return PHB_OK;
 	const StateLayout SL = stateLayout(dom, 1);
 	CcgArgs<T, D> a = {};
 	a.dom = Dom<double, D>(*dom);

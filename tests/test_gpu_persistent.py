@@ -135,3 +135,35 @@ def test_more_systems_than_a_cta_keeps_states_of_are_refused(cuda, kind, nrhs, i
     A = dom._P_st if kind == CG else dom._C_st
     with pytest.raises(RuntimeError, match="too many systems"):
         _solve(dom, kind, nrhs, A, b, 1e-6, 10, 2)
+
+
+def test_a_batch_of_more_clusters_than_fit_at_a_time(cuda):
+    """127 instances of one tile and one of 25: clusters are sized for 25 tiles, so that few are resident,
+    and 19 waves of them take 2.4 times the grid kernel's time. The default must not be that slow (the
+    bits are the same either way)."""
+    doms = []
+    for k in range(128):
+        m = hartmann_2d(*((24 + k % 8, 20 + k % 11) if k < 127 else (160, 160)))
+        seeded_state(m, k, scale=0.2)
+        m.PrepareSolve()
+        doms.append(m)
+    batch = pb.DomainBatch(doms)
+    _assemble(batch, 3)
+    b = _rhs(batch, batch.numCells(), 1, 3)
+
+    def run(ctas):
+        s = solver_for(batch, CG, torch.float64, 1, tag=f"w{ctas}")
+        best = float("inf")
+        for _ in range(5):
+            x = torch.zeros_like(b)
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            s.solve(batch._P_st, b, x, 1e-200, 40, use_graph=2, ctas_per_sm=ctas)
+            e1.record()
+            e1.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return x, best
+
+    (x0, t0), (x1, t1) = run(0), run(3)
+    assert torch.equal(x0, x1)
+    assert t0 < 1.5 * t1, (t0, t1)
