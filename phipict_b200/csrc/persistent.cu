@@ -395,12 +395,11 @@ __global__ void __launch_bounds__(PHB_TILE * cgGroups<T, D, K>(), 1) kCgPersiste
 	cgPersistentBody<T, D, K, STOPSTART>(dom, blocks, A, b, x, r, p0, p1, q, xbest, st, partial, ctrl, tol, returnBest, maxit);
 }
 
-template <typename T, int D, int K>
-__global__ void __launch_bounds__(PHB_TILE *BICG_GROUPS, 1) kBicgPersistent(Dom<double, D> dom, const BlockTab *blocks, const T *__restrict__ A, const T *__restrict__ b,
+template <typename T, int D, int K, int G = BICG_GROUPS>
+__global__ void __launch_bounds__(PHB_TILE *G, 1) kBicgPersistent(Dom<double, D> dom, const BlockTab *blocks, const T *__restrict__ A, const T *__restrict__ b,
 		T *__restrict__ x, T *__restrict__ r, T *__restrict__ r0, T *__restrict__ p0, T *__restrict__ p1, T *__restrict__ v0,
 		T *__restrict__ v1, T *__restrict__ t, SysState *st, double *partial, Control *ctrl, phb_tolerance tol, int maxit) {
 	extern __shared__ __align__(16) SysState sst[];
-	constexpr int G = BICG_GROUPS;
 	__shared__ int2 items[G][TILE_ITEMS];
 	__shared__ __align__(16) T stage[G][PHB_TILE_CELLS];
 	__shared__ double sums[G][TILE_SUMS * 3 * K * NWARPS];
@@ -639,11 +638,21 @@ int launchPersistent(const phb_domain *dom, const phb_solve *sv, cudaStream_t s,
 	}
 	T *r = (T *)(w + L.off[0]), *r0 = (T *)(w + L.off[1]), *p0 = (T *)(w + L.off[2]), *p1 = (T *)(w + L.off[3]);
 	T *v0 = (T *)(w + L.off[4]), *v1 = (T *)(w + L.off[5]), *t = (T *)(w + L.off[6]);
-	auto kern = kBicgPersistent<T, D, K>;
-	const int rc2 = configure((const void *)kern, BICG_GROUPS);
-	if (rc2) return rc2;
-	PHB_CUDA(cudaLaunchKernelEx(&cfg, kern, dm, tabs, A, b, x, r, r0, p0, p1, v0, v1, t, st, partial, ctrl, sv->tol, maxit));
-	return PHB_OK;
+	auto launch = [&](auto kern) -> int {
+		const int rc2 = configure((const void *)kern, BICG_GROUPS);
+		if (rc2) return rc2;
+		PHB_CUDA(cudaLaunchKernelEx(&cfg, kern, dm, tabs, A, b, x, r, r0, p0, p1, v0, v1, t, st, partial, ctrl, sv->tol, maxit));
+		return PHB_OK;
+	};
+	// float64 with three right-hand sides needs more than the 128 registers of two groups (it spills 456 bytes):
+	// a grid of one group per SM (one tile per SM or less) takes the kernel that may have twice as many: 32^3
+	// cells 32 -> 26 us per iteration, 48^3 35 -> 28
+	if constexpr (std::is_same<T, double>::value && K == 3) {
+		int groups = 1, ctas = 1;
+		persistentGrid(dom->ntiles, BICG_GROUPS, sv->ctas_per_sm, groups, ctas);
+		if (groups == 1) return launch(kBicgPersistent<T, D, K, 1>);
+	}
+	return launch(kBicgPersistent<T, D, K>);
 }
 #define PHB_PERSISTENT(T, D, K) template int launchPersistent<T, D, K>(const phb_domain *, const phb_solve *, cudaStream_t, bool, int);
 PHB_PERSISTENT(double, 2, 1)
