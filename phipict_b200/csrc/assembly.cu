@@ -13,6 +13,7 @@
 #include "phb_nonortho.cuh"
 #include "phb_upwind.cuh"
 #include "phb_faces.cuh"
+#include <algorithm>
 #include <initializer_list>
 
 namespace phb {
@@ -20,8 +21,21 @@ namespace phb {
 // CTAs per SM that the register budget of the branch-free kernels allows: a 3D float64 cell has 55
 // loads in flight (128 registers; at three CTAs the matrix on 192^3 took 484 instead of 351 us), the
 // others fit 85 (1999x1501 float32: 69 instead of 83 us).
-template <typename S, int D>
-constexpr int asmCtas() { return sizeof(S) == 8 && D == 3 ? 2 : 3; }
+enum AsmKernel { K_ADV_MATRIX, K_ADV_RHS, K_P_MATRIX, K_HBYA, K_DIVERGENCE, K_CORRECT, K_UXB, K_EPOT };
+template <AsmKernel K, typename S, int D, int PARTS>
+constexpr int asmCtas() {
+	if (K == K_ADV_RHS || K == K_CORRECT) return 4;
+	if (K == K_P_MATRIX || K == K_HBYA) return 3;
+	return sizeof(S) == 8 && D == 3 ? 2 : 3;
+}
+// Least use of the rounds of whole tiles in 3D (tileShare; 0: never strided, kernels of few loads that lose by it).
+// 4 blocks of 64^3 use 0.865 of them: float64 potential right-hand side 63.5 us on whole, 57.3 on strided quarter tiles,
+// float32 velocity correction 25.6 and 27.6; 96^3 float32 advection right-hand side 32.8 and 34.8.
+template <AsmKernel K, typename S, int D>
+constexpr int asmLeast() {
+	if (D != 3 || K == K_ADV_RHS || K == K_P_MATRIX || K == K_CORRECT || (K == K_UXB && sizeof(S) == 4)) return 0;
+	return sizeof(S) == 8 && K != K_HBYA ? 88 : 85;
+}
 
 // PISO_build_matrix (piso/advection.cu:27-305): implicit Euler advection-diffusion row
 // divided by the cell determinant; Adiag = its diagonal. SCALAR: the matrix of passive-scalar
@@ -115,19 +129,19 @@ __global__ void __launch_bounds__(PHB_TILE) kAdvectionMatrix(Dom<S, D> dom, cons
 // The central, orthogonal matrix (no cross terms, no upwinding): same arithmetic, all loads of a
 // cell in flight together, several tiles per CTA (phb_faces.cuh). 192^3 float64: 522 -> 347 us (196 B
 // a cell, 0.62 of HBM counting the ten transform values it uses), 1999x1501 float32: 101 -> 66 us.
-template <typename S, int D, bool SCALAR>
-__global__ void __launch_bounds__(PHB_TILE, (asmCtas<S, D>())) kAdvectionMatrixCentral(Dom<S, D> dom, const S *__restrict__ u, S *__restrict__ C,
+template <typename S, int D, bool SCALAR, int PARTS>
+__global__ void __launch_bounds__(PHB_TILE, (asmCtas<K_ADV_MATRIX, S, D, PARTS>())) kAdvectionMatrixCentral(Dom<S, D> dom, int run, const S *__restrict__ u, S *__restrict__ C,
 		S *__restrict__ Adiag, float *__restrict__ Clo, ScalarView sv, int channel) {
 	__shared__ int32_t sB[PHB_BREC];
 	__shared__ FaceMap sF[6];
-	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
+	forTiles<PARTS, S, D>(dom, run, sB, sF, [&](int l0_, int nc_, int j0_, auto aligned) {
 		constexpr bool SAME = decltype(aligned)::value;
 		const int inst = sB[B_INST];
 		const S dt = S(dom.dt[inst]);
 		const S nu = SCALAR ? S(scalarNu(sv, channel, dom.nu[inst])) : S(dom.nu[inst]);
 		const int64_t N = dom.ncells;
 		const Comps<S, D> uc(sB, u);
-		for (int j_ = 0; j_ < CPT; ++j_) {
+		for (int j_ = j0_; j_ < j0_ + CPT / PARTS; ++j_) {
 			Cell c;
 			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
 			const Faces<D> n = cellFaces<D>(sB, sF, c);
@@ -256,20 +270,18 @@ __global__ void __launch_bounds__(PHB_TILE, sizeof(S) == 8 ? 2 : 3) kAdvectionRh
 }
 
 // The same for the central scheme, one cell at a time: a streaming kernel, its few cells on fixed
-// faces corrected after the loads. 192^3 float64: 245 us with a CTA per tile, 171 with several.
-template <typename S, int D>
-__global__ void __launch_bounds__(PHB_TILE, 4) kAdvectionRhsCentral(Dom<S, D> dom, const S *__restrict__ u, const S *__restrict__ src,
+// faces corrected after the loads. 192^3 float64: 229 us in the form above, 154 here.
+template <typename S, int D, int PARTS>
+__global__ void __launch_bounds__(PHB_TILE, (asmCtas<K_ADV_RHS, S, D, PARTS>())) kAdvectionRhsCentral(Dom<S, D> dom, int run, const S *__restrict__ u, const S *__restrict__ src,
 		int srcMode, S *__restrict__ rhs) {
 	__shared__ int32_t sB[PHB_BREC];
 	__shared__ FaceMap sF[6];
-	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
-		constexpr bool SAME = decltype(aligned)::value;
+	forTiles<PARTS, S, D>(dom, run, sB, sF, [&](int l0_, int nc_, int j0_, auto) {
 		const int inst = sB[B_INST];
 		const S dt = S(dom.dt[inst]);
 		const S nu = S(dom.nu[inst]);
-#pragma unroll 2
 		const Comps<S, D> uc(sB, u);
-		for (int j_ = 0; j_ < CPT; ++j_) {
+		for (int j_ = j0_; j_ < j0_ + CPT / PARTS; ++j_) {
 			Cell c;
 			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
 			S uv[D], sv[D], bs[D];
@@ -456,15 +468,15 @@ __global__ void __launch_bounds__(PHB_TILE) kLaplaceMatrix(Dom<S, D> dom, const 
 
 // The pressure matrix without cross terms: same arithmetic, all loads of a cell in flight together.
 // 192^3 float64: 261 -> 229 us (0.69 of HBM).
-template <typename S, int D>
-__global__ void __launch_bounds__(PHB_TILE, 3) kPressureMatrix(Dom<S, D> dom, const S *__restrict__ Adiag, S *__restrict__ P,
+template <typename S, int D, int PARTS>
+__global__ void __launch_bounds__(PHB_TILE, (asmCtas<K_P_MATRIX, S, D, PARTS>())) kPressureMatrix(Dom<S, D> dom, int run, const S *__restrict__ Adiag, S *__restrict__ P,
 		float *__restrict__ Plo) {
 	__shared__ int32_t sB[PHB_BREC];
 	__shared__ FaceMap sF[6];
-	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
+	forTiles<PARTS, S, D>(dom, run, sB, sF, [&](int l0_, int nc_, int j0_, auto aligned) {
 		constexpr bool SAME = decltype(aligned)::value;
 		const int64_t N = dom.ncells;
-		for (int j_ = 0; j_ < CPT; ++j_) {
+		for (int j_ = j0_; j_ < j0_ + CPT / PARTS; ++j_) {
 			Cell c;
 			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
 			const Faces<D> n = cellFaces<D>(sB, sF, c);
@@ -664,19 +676,18 @@ __global__ void __launch_bounds__(PHB_TILE, sizeof(S) == 8 ? 2 : 3) kPressureRhs
 
 // HbyA of the central scheme, one cell at a time with all its loads in flight together: the row form
 // above resolves the faces of the quads that touch one (192^3 float64: 585 us in that form, 408 here).
-template <typename S, int D>
-__global__ void __launch_bounds__(PHB_TILE, 3) kPressureRhsCentral(Dom<S, D> dom, const S *__restrict__ C, const S *__restrict__ Adiag,
+template <typename S, int D, int PARTS>
+__global__ void __launch_bounds__(PHB_TILE, (asmCtas<K_HBYA, S, D, PARTS>())) kPressureRhsCentral(Dom<S, D> dom, int run, const S *__restrict__ C, const S *__restrict__ Adiag,
 		const S *__restrict__ u, const S *__restrict__ ustar, const S *__restrict__ src, int srcMode, S *__restrict__ hbya) {
 	__shared__ int32_t sB[PHB_BREC];
 	__shared__ FaceMap sF[6];
-	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
-		constexpr bool SAME = decltype(aligned)::value;
+	forTiles<PARTS, S, D>(dom, run, sB, sF, [&](int l0_, int nc_, int j0_, auto) {
 		const int inst = sB[B_INST];
 		const S dt = S(dom.dt[inst]);
 		const S nu = S(dom.nu[inst]);
 		const int64_t N = dom.ncells;
 		const Comps<S, D> usc(sB, ustar), uc(sB, u);
-		for (int j_ = 0; j_ < CPT; ++j_) {
+		for (int j_ = j0_; j_ < j0_ + CPT / PARTS; ++j_) {
 			Cell c;
 			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
 			const Faces<D> n = cellFaces<D>(sB, sF, c);
@@ -715,14 +726,14 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kPressureRhsCentral(Dom<S, D> dom
 
 // k_computePressureRHSdivergenceFromFlux (pressure.cu:756-801), no face transforms (192^3 float64:
 // 275 -> 229 us, 0.54 of HBM: 55 loads a cell, most of them L1 hits, bound the issue)
-template <typename S, int D>
-__global__ void __launch_bounds__(PHB_TILE, (asmCtas<S, D>())) kDivergence(Dom<S, D> dom, const S *__restrict__ field, S *__restrict__ div) {
+template <typename S, int D, int PARTS>
+__global__ void __launch_bounds__(PHB_TILE, (asmCtas<K_DIVERGENCE, S, D, PARTS>())) kDivergence(Dom<S, D> dom, int run, const S *__restrict__ field, S *__restrict__ div) {
 	__shared__ int32_t sB[PHB_BREC];
 	__shared__ FaceMap sF[6];
-	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
+	forTiles<PARTS, S, D>(dom, run, sB, sF, [&](int l0_, int nc_, int j0_, auto aligned) {
 		constexpr bool SAME = decltype(aligned)::value;
 		const Comps<S, D> fc(sB, field);
-		for (int j_ = 0; j_ < CPT; ++j_) {
+		for (int j_ = j0_; j_ < j0_ + CPT / PARTS; ++j_) {
 			Cell c;
 			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
 			S fl[2 * D];
@@ -737,14 +748,13 @@ __global__ void __launch_bounds__(PHB_TILE, (asmCtas<S, D>())) kDivergence(Dom<S
 
 // PISO_update_velocity, version 1 (velocity_correction.cu:27-60) with the finite
 // difference gradient of getPressureGradient (piso/device/velocity.cuh:347-378)
-template <typename S, int D>
-__global__ void __launch_bounds__(PHB_TILE, 4) kCorrectVelocity(Dom<S, D> dom, const S *__restrict__ p, const S *__restrict__ hbya,
+template <typename S, int D, int PARTS>
+__global__ void __launch_bounds__(PHB_TILE, (asmCtas<K_CORRECT, S, D, PARTS>())) kCorrectVelocity(Dom<S, D> dom, int run, const S *__restrict__ p, const S *__restrict__ hbya,
 		const S *__restrict__ Adiag, S *__restrict__ u) {
 	__shared__ int32_t sB[PHB_BREC];
 	__shared__ FaceMap sF[6];
-	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
-		constexpr bool SAME = decltype(aligned)::value;
-		for (int j_ = 0; j_ < CPT; ++j_) {
+	forTiles<PARTS, S, D>(dom, run, sB, sF, [&](int l0_, int nc_, int j0_, auto) {
+		for (int j_ = j0_; j_ < j0_ + CPT / PARTS; ++j_) {
 			Cell c;
 			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
 			const Faces<D> n = cellFaces<D>(sB, sF, c);
@@ -812,15 +822,15 @@ __device__ __forceinline__ void epotDirichlet(const Dom<S, D> &dom, const Cell &
 }
 
 // u x e_b fused with k_computeEpotRHS (mhd/potential.cu:273-323)
-template <typename S, int D>
-__global__ void __launch_bounds__(PHB_TILE, (asmCtas<S, D>())) kUxbEpotRhs(Dom<S, D> dom, const S *__restrict__ u, const double *__restrict__ eb,
+template <typename S, int D, int PARTS>
+__global__ void __launch_bounds__(PHB_TILE, (asmCtas<K_UXB, S, D, PARTS>())) kUxbEpotRhs(Dom<S, D> dom, int run, const S *__restrict__ u, const double *__restrict__ eb,
 		S *__restrict__ uxb, S *__restrict__ rhs) {
 	__shared__ int32_t sB[PHB_BREC];
 	__shared__ FaceMap sF[6];
-	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
+	forTiles<PARTS, S, D>(dom, run, sB, sF, [&](int l0_, int nc_, int j0_, auto aligned) {
 		constexpr bool SAME = decltype(aligned)::value;
 		const double *e = eb + 3 * sB[B_INST];
-		for (int j_ = 0; j_ < CPT; ++j_) {
+		for (int j_ = j0_; j_ < j0_ + CPT / PARTS; ++j_) {
 			Cell c;
 			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
 			const Faces<D> n = cellFaces<D>(sB, sF, c);
@@ -849,14 +859,14 @@ __global__ void __launch_bounds__(PHB_TILE, (asmCtas<S, D>())) kUxbEpotRhs(Dom<S
 }
 
 // k_computeEpotRHS (mhd/potential.cu:273-323) of a given in-plane field [inst][dims][cells]
-template <typename S, int D>
-__global__ void __launch_bounds__(PHB_TILE, (asmCtas<S, D>())) kEpotRhs(Dom<S, D> dom, const S *__restrict__ field, S *__restrict__ rhs) {
+template <typename S, int D, int PARTS>
+__global__ void __launch_bounds__(PHB_TILE, (asmCtas<K_EPOT, S, D, PARTS>())) kEpotRhs(Dom<S, D> dom, int run, const S *__restrict__ field, S *__restrict__ rhs) {
 	__shared__ int32_t sB[PHB_BREC];
 	__shared__ FaceMap sF[6];
-	forTiles<S, D>(dom, sB, sF, [&](int l0_, int nc_, auto aligned) {
+	forTiles<PARTS, S, D>(dom, run, sB, sF, [&](int l0_, int nc_, int j0_, auto aligned) {
 		constexpr bool SAME = decltype(aligned)::value;
 		const Comps<S, D> fc(sB, field);
-		for (int j_ = 0; j_ < CPT; ++j_) {
+		for (int j_ = j0_; j_ < j0_ + CPT / PARTS; ++j_) {
 			Cell c;
 			if (!cellAt<D>(sB, l0_, nc_, j_, c)) return;
 			const Faces<D> n = cellFaces<D>(sB, sF, c);
@@ -1037,7 +1047,13 @@ using namespace phb;
 		else return setError(PHB_ERR_ARG, "unsupported dims/dtype");                                \
 	} while (0)
 
-#define PHB_RESIDENT(DOM, KERN) tileGrid<KERN>((DOM)->ntiles), dim3(PHB_TILE), 0, (cudaStream_t)stream
+// Launch the form of a kernel that tileShare chooses
+#define PHB_SHARED(DOM, KIND, WHOLE, QUARTER, ...) \
+	do { \
+		const TileShare ts_ = tileShare<WHOLE, QUARTER>(DOM, asmLeast<KIND, S, D>()); \
+		if (ts_.quarters) QUARTER<<<ts_.ctas, PHB_TILE, 0, (cudaStream_t)stream>>>(Dom<S, D>(*(DOM)), ts_.run, __VA_ARGS__); \
+		else WHOLE<<<ts_.ctas, PHB_TILE, 0, (cudaStream_t)stream>>>(Dom<S, D>(*(DOM)), ts_.run, __VA_ARGS__); \
+	} while (0)
 #define PHB_TILES(DOM) dim3((DOM)->ntiles), dim3(PHB_TILE), 0, (cudaStream_t)stream
 
 // The device view of a launch whose quad kernels may use vector loads: every field operand
@@ -1062,8 +1078,8 @@ extern "C" int phb_advection_matrix(const phb_domain *dom, const void *u, void *
 		return checkLaunch("kAdvectionMatrix<non-orthogonal>");
 	}
 	if (dom->scheme == 0)
-		PHB_DISPATCH(dom, (kAdvectionMatrixCentral<S, D, false><<<PHB_RESIDENT(dom, (kAdvectionMatrixCentral<S, D, false>))>>>(Dom<S, D>(*dom), (const S *)u, (S *)C, (S *)Adiag, C_lo,
-			ScalarView{}, 0)));
+		PHB_DISPATCH(dom, PHB_SHARED(dom, K_ADV_MATRIX, (kAdvectionMatrixCentral<S, D, false, 1>), (kAdvectionMatrixCentral<S, D, false, CPT>), (const S *)u, (S *)C, (S *)Adiag, C_lo,
+			ScalarView{}, 0));
 	else
 		PHB_DISPATCH(dom, kAdvectionMatrix<S, D><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)u, (S *)C, (S *)Adiag, C_lo));
 	return checkLaunch("kAdvectionMatrix");
@@ -1082,8 +1098,8 @@ extern "C" int phb_scalar_matrix(const phb_domain *dom, const void *u, const phb
 		return checkLaunch("kAdvectionMatrix<scalar, non-orthogonal>");
 	}
 	if (dom->scheme == 0)
-		PHB_DISPATCH(dom, (kAdvectionMatrixCentral<S, D, true><<<PHB_RESIDENT(dom, (kAdvectionMatrixCentral<S, D, true>))>>>(Dom<S, D>(*dom), (const S *)u, (S *)C, (S *)Adiag, C_lo, sv,
-			channel)));
+		PHB_DISPATCH(dom, PHB_SHARED(dom, K_ADV_MATRIX, (kAdvectionMatrixCentral<S, D, true, 1>), (kAdvectionMatrixCentral<S, D, true, CPT>), (const S *)u, (S *)C, (S *)Adiag, C_lo, sv,
+			channel));
 	else
 		PHB_DISPATCH(dom, kAdvectionMatrix<S, D, true><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)u, (S *)C, (S *)Adiag, C_lo, sv, channel));
 	return checkLaunch("kAdvectionMatrix<scalar>");
@@ -1105,8 +1121,8 @@ extern "C" int phb_advection_rhs(const phb_domain *dom, const void *u, const voi
 		PHB_DISPATCH(dom, (kAdvectionRhs<S, D><<<PHB_TILES(dom)>>>(quadView<S, D>(dom, {u, src, rhs}), (const S *)u, (const S *)src,
 			src_mode, (S *)rhs)));
 	else
-		PHB_DISPATCH(dom, (kAdvectionRhsCentral<S, D><<<PHB_RESIDENT(dom, (kAdvectionRhsCentral<S, D>))>>>(Dom<S, D>(*dom), (const S *)u,
-			(const S *)src, src_mode, (S *)rhs)));
+		PHB_DISPATCH(dom, PHB_SHARED(dom, K_ADV_RHS, (kAdvectionRhsCentral<S, D, 1>), (kAdvectionRhsCentral<S, D, CPT>), (const S *)u,
+			(const S *)src, src_mode, (S *)rhs));
 	return checkLaunch("kAdvectionRhs");
 }
 extern "C" int phb_pressure_matrix(const phb_domain *dom, const void *Adiag, void *P, float *P_lo, phb_stream stream) {
@@ -1116,7 +1132,7 @@ extern "C" int phb_pressure_matrix(const phb_domain *dom, const void *Adiag, voi
 		PHB_DISPATCH(dom, (kLaplaceMatrix<S, D, false, true><<<PHB_TILES(dom)>>>(Dom<S, D>(*dom), (const S *)Adiag, (S *)P, P_lo)));
 		return checkLaunch("kLaplaceMatrix<non-orthogonal>");
 	}
-	PHB_DISPATCH(dom, (kPressureMatrix<S, D><<<PHB_RESIDENT(dom, (kPressureMatrix<S, D>))>>>(Dom<S, D>(*dom), (const S *)Adiag, (S *)P, P_lo)));
+	PHB_DISPATCH(dom, PHB_SHARED(dom, K_P_MATRIX, (kPressureMatrix<S, D, 1>), (kPressureMatrix<S, D, CPT>), (const S *)Adiag, (S *)P, P_lo));
 	return checkLaunch("kPressureMatrix");
 }
 extern "C" int phb_epot_matrix(const phb_domain *dom, void *E, float *E_lo, phb_stream stream) {
@@ -1134,26 +1150,26 @@ extern "C" int phb_pressure_rhs(const phb_domain *dom, const void *C, const void
 		PHB_DISPATCH(dom, (kPressureRhs<S, D><<<PHB_TILES(dom)>>>(quadView<S, D>(dom, {C, Adiag, u, ustar, src, hbya}),
 			(const S *)C, (const S *)Adiag, (const S *)u, (const S *)ustar, (const S *)src, src_mode, (S *)hbya)));
 	else
-		PHB_DISPATCH(dom, (kPressureRhsCentral<S, D><<<PHB_RESIDENT(dom, (kPressureRhsCentral<S, D>))>>>(Dom<S, D>(*dom), (const S *)C, (const S *)Adiag, (const S *)u,
-			(const S *)ustar, (const S *)src, src_mode, (S *)hbya)));
+		PHB_DISPATCH(dom, PHB_SHARED(dom, K_HBYA, (kPressureRhsCentral<S, D, 1>), (kPressureRhsCentral<S, D, CPT>), (const S *)C, (const S *)Adiag, (const S *)u,
+			(const S *)ustar, (const S *)src, src_mode, (S *)hbya));
 	return checkLaunch("kPressureRhs");
 }
 extern "C" int phb_divergence(const phb_domain *dom, const void *field, void *div, phb_stream stream) {
 	if (!dom || !field || !div) return setError(PHB_ERR_ARG, "phb_divergence: null argument");
 	if (dom->ntiles == 0) return PHB_OK;
-	PHB_DISPATCH(dom, kDivergence<S, D><<<PHB_RESIDENT(dom, (kDivergence<S, D>))>>>(Dom<S, D>(*dom), (const S *)field, (S *)div));
+	PHB_DISPATCH(dom, PHB_SHARED(dom, K_DIVERGENCE, (kDivergence<S, D, 1>), (kDivergence<S, D, CPT>), (const S *)field, (S *)div));
 	return checkLaunch("kDivergence");
 }
 extern "C" int phb_correct_velocity(const phb_domain *dom, const void *p, const void *hbya, const void *Adiag, void *u, phb_stream stream) {
 	if (!dom || !p || !hbya || !Adiag || !u) return setError(PHB_ERR_ARG, "phb_correct_velocity: null argument");
 	if (dom->ntiles == 0) return PHB_OK;
-	PHB_DISPATCH(dom, kCorrectVelocity<S, D><<<PHB_RESIDENT(dom, (kCorrectVelocity<S, D>))>>>(Dom<S, D>(*dom), (const S *)p, (const S *)hbya, (const S *)Adiag, (S *)u));
+	PHB_DISPATCH(dom, PHB_SHARED(dom, K_CORRECT, (kCorrectVelocity<S, D, 1>), (kCorrectVelocity<S, D, CPT>), (const S *)p, (const S *)hbya, (const S *)Adiag, (S *)u));
 	return checkLaunch("kCorrectVelocity");
 }
 extern "C" int phb_uxb_epot_rhs(const phb_domain *dom, const void *u, const double *e_b, void *uxb, void *rhs, phb_stream stream) {
 	if (!dom || !u || !e_b || !uxb || !rhs) return setError(PHB_ERR_ARG, "phb_uxb_epot_rhs: null argument");
 	if (dom->ntiles == 0) return PHB_OK;
-	PHB_DISPATCH(dom, kUxbEpotRhs<S, D><<<PHB_RESIDENT(dom, (kUxbEpotRhs<S, D>))>>>(Dom<S, D>(*dom), (const S *)u, e_b, (S *)uxb, (S *)rhs));
+	PHB_DISPATCH(dom, PHB_SHARED(dom, K_UXB, (kUxbEpotRhs<S, D, 1>), (kUxbEpotRhs<S, D, CPT>), (const S *)u, e_b, (S *)uxb, (S *)rhs));
 	return checkLaunch("kUxbEpotRhs");
 }
 extern "C" int phb_current_lorentz(const phb_domain *dom, const void *phi, const void *uxb, const double *e_b,
@@ -1167,7 +1183,7 @@ extern "C" int phb_current_lorentz(const phb_domain *dom, const void *phi, const
 extern "C" int phb_epot_rhs(const phb_domain *dom, const void *field, void *rhs, phb_stream stream) {
 	if (!dom || !field || !rhs) return setError(PHB_ERR_ARG, "phb_epot_rhs: null argument");
 	if (dom->ntiles == 0) return PHB_OK;
-	PHB_DISPATCH(dom, kEpotRhs<S, D><<<PHB_RESIDENT(dom, (kEpotRhs<S, D>))>>>(Dom<S, D>(*dom), (const S *)field, (S *)rhs));
+	PHB_DISPATCH(dom, PHB_SHARED(dom, K_EPOT, (kEpotRhs<S, D, 1>), (kEpotRhs<S, D, CPT>), (const S *)field, (S *)rhs));
 	return checkLaunch("kEpotRhs");
 }
 extern "C" int phb_nonortho_rhs(const phb_domain *dom, int kind, const void *field, const phb_scalar *sc, const void *Adiag,

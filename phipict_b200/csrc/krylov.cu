@@ -758,7 +758,7 @@ __global__ void __launch_bounds__(PHB_TILE, 3) kStencilApply(Dom<double, D> dom,
 	__shared__ FaceMap sF[6];
 	const int64_t N = dom.ncells;
 	constexpr int J = 2;
-	forTiles<double, D>(dom, sB, sF, [&](int l0, int nc, auto) {
+	forTiles<1, double, D>(dom, 0, sB, sF, [&](int l0, int nc, int, auto) {
 	for (int j0 = 0; j0 < CPT; j0 += J) {
 		int g[J], o[J][2 * D];
 		unsigned int fixed[J];
@@ -1045,8 +1045,8 @@ extern "C" int phb_stencil_apply(const phb_domain *dom, const double *A, const d
 	if (dom->dims != 2 && dom->dims != 3) return setError(PHB_ERR_ARG, "phb_stencil_apply: dims");
 	if (dom->ntiles == 0) return PHB_OK;
 	cudaStream_t s = (cudaStream_t)stream;
-	if (dom->dims == 2) kStencilApply<2><<<tileGrid<kStencilApply<2>>(dom->ntiles), PHB_TILE, 0, s>>>(Dom<double, 2>(*dom), A, X, Y, nvec, stride);
-	else kStencilApply<3><<<tileGrid<kStencilApply<3>>(dom->ntiles), PHB_TILE, 0, s>>>(Dom<double, 3>(*dom), A, X, Y, nvec, stride);
+	if (dom->dims == 2) kStencilApply<2><<<std::min(dom->ntiles, residentCtas<kStencilApply<2>>()), PHB_TILE, 0, s>>>(Dom<double, 2>(*dom), A, X, Y, nvec, stride);
+	else kStencilApply<3><<<std::min(dom->ntiles, residentCtas<kStencilApply<3>>()), PHB_TILE, 0, s>>>(Dom<double, 3>(*dom), A, X, Y, nvec, stride);
 	return checkLaunch("kStencilApply");
 }
 

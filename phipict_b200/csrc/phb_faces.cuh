@@ -9,6 +9,7 @@
 // one another.
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 #include "phb_device.cuh"
 
@@ -60,22 +61,30 @@ __device__ __forceinline__ void buildFaceMap(const Dom<S, D> &dom, const int32_t
 	m.cx = cf[0]; m.cy = cf[1]; m.cz = cf[2];
 }
 
-// Visit tiles blockIdx.x, blockIdx.x + gridDim.x, ... : f(first cell, cells of the block, aligned) with
-// the block record and its face maps staged; aligned: no face of the block maps its axis to another
-// component (compile-time components make half the index arithmetic). A CTA takes several tiles (the grid is the CTAs that fit
-// the chip, tileGrid): a CTA per tile spends more than half its life on the reads that lead to its
-// first cell (tile, block record, instance parameters); here they are made once per block.
-template <typename S, int D, typename F>
-__device__ __forceinline__ void forTiles(const Dom<S, D> &dom, int32_t *sB, FaceMap *sF, F f) {
+// Visit the CTA's share of the tiles: f(first cell of the tile, cells of the block, first of its cells per
+// thread, aligned) with the block record and its face maps staged; aligned: no face of the block maps its axis to
+// another component (compile-time components make half the index arithmetic). A CTA takes several (the grid is
+// the CTAs that fit the chip): a CTA per tile spends more than half its life on the reads that lead to its first
+// cell (tile, block record, instance parameters); here they are made once per block. PARTS = 1: whole tiles;
+// PARTS = CPT: quarter tiles of a cell per thread, `run` consecutive ones per CTA or (run 0) gridDim.x apart
+// (tileShare chooses).
+template <int PARTS, typename S, int D, typename F>
+__device__ __forceinline__ void forTiles(const Dom<S, D> &dom, int run, int32_t *sB, FaceMap *sF, F f) {
+	static_assert(PARTS == 1 || PARTS == CPT, "whole or quarter tiles");
 	int staged = -1; // the block in sB (uniform over the CTA)
 	bool aligned = false;
+	const int items = dom.ntiles * PARTS;
+	const bool row = PARTS != 1 && run > 0;
+	const int step = row ? 1 : int(gridDim.x);
+	const int first = row ? int(blockIdx.x) * run : int(blockIdx.x);
+	const int end = row ? min(items, first + run) : items;
 	int b = 0, l0 = 0;
-	if (int(blockIdx.x) < dom.ntiles) {
-		b = __ldg(dom.tiles + 2 * blockIdx.x);
-		l0 = __ldg(dom.tiles + 2 * blockIdx.x + 1);
+	if (first < end) {
+		b = __ldg(dom.tiles + 2 * (first / PARTS));
+		l0 = __ldg(dom.tiles + 2 * (first / PARTS) + 1);
 	}
-	for (int t = blockIdx.x; t < dom.ntiles; t += gridDim.x) {
-		const int n = t + int(gridDim.x) < dom.ntiles ? t + int(gridDim.x) : t;
+	for (int t = first; t < end; t += step) {
+		const int n = (t + step < end ? t + step : t) / PARTS;
 		const int bn = __ldg(dom.tiles + 2 * n), ln = __ldg(dom.tiles + 2 * n + 1); // the next tile
 		if (b != staged) {
 			__syncthreads();
@@ -90,16 +99,32 @@ __device__ __forceinline__ void forTiles(const Dom<S, D> &dom, int32_t *sB, Face
 			staged = b;
 		}
 		const int nc = sB[B_NX] * sB[B_NY] * (D > 2 ? sB[B_NZ] : 1);
-		if (aligned) f(l0, nc, std::true_type{});
-		else f(l0, nc, std::false_type{});
+		const int j0 = PARTS == 1 ? 0 : t % PARTS;
+		if (aligned) f(l0, nc, j0, std::true_type{});
+		else f(l0, nc, j0, std::false_type{});
 		b = bn;
 		l0 = ln;
 	}
 }
 
-// The grid of such a kernel: as many CTAs as the device holds at once, at most one per tile.
+// How a launch shares out its tiles: a kernel has a form for whole and one for quarter tiles.
+// - Quarter tiles in runs, where whole tiles would give most CTAs one or none (a thread then walks its four
+//   cells one after the other while most of the chip idles) or leave the last of a few rounds nearly empty: where the
+//   longest run is at most three quarters (kernels of few loads, `least` 0, and 2D: five eighths) of the cells that a
+//   thread of the whole form takes, up to MAX_RUN. 64 x 32 cells float32: matrix 14.3 -> 9.2 us, HbyA 17.4 -> 9.3;
+//   32^3 float64: HbyA 38 -> 17; 432 tiles float64 on 296 CTAs: potential right-hand side 35.8 -> 29.7. Three
+//   quarters where five eighths are the rule: 2D divergence, 256 tiles, 8.4 -> 10.2; 96^3 float32 advection
+//   right-hand side 26.8 -> 29.7.
+// - Quarter tiles gridDim.x apart, in 3D on blocks of eight tiles and more (runs meet fewer blocks), where whole
+//   tiles would use less than `least` percent of their rounds: 99 x 101 x 97 float64, 948 tiles in 4 rounds of
+//   296: matrix 74.7 -> 64.5 us, HbyA 85 -> 67.
+// - Whole tiles otherwise: fewer reads of tile records, four cells' index arithmetic unrolled.
+struct TileShare {
+	bool quarters;
+	int ctas, run;
+};
 template <auto KERN>
-inline dim3 tileGrid(int ntiles) {
+inline int residentCtas() { // CTAs of a kernel that the device holds at a time
 	static const int resident = [] {
 		int dev = 0, sms = 0, per = 0;
 		if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
@@ -109,7 +134,17 @@ inline dim3 tileGrid(int ntiles) {
 		}
 		return per * sms;
 	}();
-	return dim3(ntiles < resident ? ntiles : resident);
+	return resident;
+}
+template <auto WHOLE, auto QUARTER>
+inline TileShare tileShare(const phb_domain *dom, int least) {
+	constexpr int MAX_RUN = 6;
+	const int64_t tiles = dom->ntiles, quarter = residentCtas<QUARTER>(), whole = residentCtas<WHOLE>();
+	const int64_t rounds = (tiles + whole - 1) / whole, run = (tiles * CPT + quarter - 1) / quarter;
+	const int64_t fill = std::max<int64_t>(1, std::min<int64_t>(CPT, (dom->ncells + tiles * PHB_TILE - 1) / (tiles * PHB_TILE))); // cells of a thread
+	if (run <= MAX_RUN && 8 * run <= (least ? 6 : 5) * rounds * fill) return {true, int((tiles * CPT + run - 1) / run), int(run)};
+	if (tiles >= 8 * (int64_t)dom->nblocks && 100 * tiles < least * rounds * whole) return {true, int(std::min(quarter, tiles * CPT)), 0};
+	return {false, int(std::min(tiles, whole)), 0};
 }
 
 // The neighbours of one cell: state and metric indices, the neighbour's component across the face.

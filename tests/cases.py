@@ -150,6 +150,49 @@ def skewed_pair_2d(n=6, *, device="cuda", dtype=torch.float64, nu=0.05, seed=1):
     return dom
 
 
+def rotated_pair_3d(n=(10, 12, 8), m=14, *, swapped=False, device="cuda", dtype=torch.float64, nu=0.05, distorted=False,
+                    seed=1):
+    """Two 3D blocks whose connection turns the axes: block a (n cells) meets block b's -y face with
+    its +x face, a's y axis along b's z and a's z axis along b's x, mirrored (``swapped``: a's y along
+    b's x, mirrored, and a's z along b's z, which changes the handedness). b has m cells in y and is
+    periodic in its z. ``distorted``: seeded, sheared vertex coordinates (cross terms and differing
+    metrics on both sides; the blocks are not meant to fit together in space)."""
+    nx, ny, nz = n
+    bx, bz = (ny, nz) if swapped else (nz, ny)
+    dom = pb.Domain(3, torch.tensor([nu]), name="rot3", device=device, dtype=dtype)
+    if distorted:
+        g = torch.Generator(device="cpu").manual_seed(seed)
+
+        def coords(size, x0):
+            v = rectilinear_vertices(*(np.linspace(x0, x0 + 1.0, k + 1) for k in size), dtype=torch.float64)
+            inner = v[0, :, 1:-1, 1:-1, 1:-1]
+            inner += 0.25 / max(size) * (torch.rand(inner.shape, generator=g, dtype=torch.float64) - 0.5)
+            v[0, 0] += 0.2 * v[0, 1] + 0.1 * v[0, 2]
+            return v.to(dtype)
+
+        a = dom.CreateBlock(vertexCoordinates=coords((nx, ny, nz), 0.0), name="a")
+        b = dom.CreateBlock(vertexCoordinates=coords((bx, m, bz), 2.0), name="b")
+    else:
+        a = dom.CreateBlock(velocity=torch.zeros(1, 3, nz, ny, nx, dtype=dtype), name="a")
+        b = dom.CreateBlock(velocity=torch.zeros(1, 3, bz, m, bx, dtype=dtype), name="b")
+    a.ConnectBlock("+x", b, "-y", *(("+x", "-z") if swapped else ("-z", "+x")))
+    for f in ("-x", "-y", "+y", "-z", "+z"):
+        a.CloseBoundary(f)
+    for f in ("-x", "+x", "+y"):
+        b.CloseBoundary(f)
+    b.MakePeriodic("z")
+    return dom
+
+
+def periodic_box_3d(nx=64, ny=48, nz=48, *, device="cuda", dtype=torch.float64, nu=0.05):
+    """One block without coordinates, periodic along every axis: every face of a row is open."""
+    dom = pb.Domain(3, torch.tensor([nu]), name="box", device=device, dtype=dtype)
+    b = dom.CreateBlock(velocity=torch.zeros(1, 3, nz, ny, nx, dtype=dtype), name="box")
+    for a in "xyz":
+        b.MakePeriodic(a)
+    return dom
+
+
 def seeded_state(dom, seed=0, scale=0.3, base=(1.0,)):
     """Random block velocities (and a base flow along x)."""
     g = torch.Generator(device="cpu").manual_seed(seed)
