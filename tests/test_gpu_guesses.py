@@ -173,6 +173,45 @@ def test_stencil_apply_on_other_shapes(cuda, shape):
 
 
 @pytest.mark.gpu
+def test_stencil_apply_on_a_batch(cuda):
+    """Instances of different sizes and shapes in one launch: every instance gets the bits that it gets
+    alone."""
+    import ctypes as ct
+
+    from cases import rotated_pair_2d
+    from phipict_b200 import _C, _lib
+
+    doms = [hartmann_2d(33, 31), rotated_pair_2d(16), hartmann_2d(64, 24), hartmann_2d(7, 5), hartmann_2d(51, 53)]
+    ts = torch.tensor([1e-2], dtype=torch.float64)
+    for k, dom in enumerate(doms):
+        seeded_state(dom, k, scale=0.2)
+        dom.PrepareSolve()
+        _C.SetupAdvectionMatrix(dom, ts)
+        _C.SetupPressureMatrix(dom, ts)
+    batch = pb.DomainBatch(doms)
+    _C.SetupAdvectionMatrix(batch, ts)
+    _C.SetupPressureMatrix(batch, ts)
+    N = batch.numCells()
+    g = torch.Generator(device="cuda").manual_seed(6)
+    X = torch.randn(3, (N + 3) // 4 * 4 + 8, dtype=torch.float64, device="cuda", generator=g)
+
+    def apply(d, X):
+        Y = torch.full_like(X, float("nan"))
+        _lib.call("phb_stencil_apply", ct.byref(d.desc()), d._stencil("P").data_ptr(), X.data_ptr(), Y.data_ptr(), X.shape[0],
+                  X.stride(0), _lib.stream_ptr(X.device))
+        return Y
+
+    Y = apply(batch, X)
+    assert torch.isnan(Y[:, N:]).all()
+    for e, dom in enumerate(doms):
+        sl = batch.instance_slice(e)
+        n = dom.numCells()
+        Xe = torch.zeros(3, (n + 3) // 4 * 4, dtype=torch.float64, device="cuda")
+        Xe[:, :n] = X[:, sl]
+        assert torch.equal(apply(dom, Xe)[:, :n], Y[:, sl]), e
+
+
+@pytest.mark.gpu
 def test_projection_solve_matches_a_dense_solve(cuda):
     """phb_projection_solve against torch.linalg.solve on symmetric definite systems of both
     signs, and the coefficient 0 of a row that is linearly dependent on the others."""
