@@ -752,7 +752,7 @@ static int emitSolve(const phb_domain *dom, const phb_solve *sv, cudaStream_t s,
 // CTA that shares in the vectors) and not once per vector. What bounds it: a chain of one round trip to
 // memory per vector and cell of a thread. Two cells of a thread at a time spilled; one cell, quarter tiles
 // and the vectors of small domains shared out over CTAs: 12 rows of 442,368 cells 70 -> 51 us, of 2048 cells
-// 43 -> 8, of 2.1 M cells 295 -> 217. The centre and face terms are summed in the order of the solvers' own products.
+// 43 -> 8, of 2.1 M cells 289 -> 221. The centre and face terms are summed in the order of the solvers' own products.
 template <int D, int PARTS>
 __global__ void __launch_bounds__(PHB_TILE, 4) kStencilApply(Dom<double, D> dom, int run, const double *__restrict__ A,
 		const double *__restrict__ X, double *__restrict__ Y, int nvec, int64_t stride) {
@@ -1024,7 +1024,9 @@ extern "C" int phb_stencil_apply(const phb_domain *dom, const double *A, const d
 	cudaStream_t s = (cudaStream_t)stream;
 	auto launch = [&](auto dims) {
 		constexpr int D = decltype(dims)::value;
-		const TileShare ts = tileShare<kStencilApply<D, 1>, kStencilApply<D, CPT>>(dom, 0);
+		// longer runs of quarter tiles with more vectors (442,368 cells, whole tiles and runs of three: one vector
+		// 10.4 and 12.4 us, 12 vectors 61 and 51); never strided (the least use is 1 percent)
+		const TileShare ts = tileShare<kStencilApply<D, 1>, kStencilApply<D, CPT>>(dom, nvec >= 4 ? 1 : 0);
 		// the vectors are shared out over CTAs too where the tiles leave room for it
 		const dim3 grid(ts.ctas, std::max(1, std::min(nvec, residentCtas<kStencilApply<D, CPT>>() / ts.ctas)));
 		auto kern = ts.quarters ? kStencilApply<D, CPT> : kStencilApply<D, 1>;
