@@ -937,19 +937,21 @@ extern "C" int64_t phb_solve_state_bytes(const phb_domain *dom, int nrhs) {
 	return (int64_t)stateLayout(dom, nrhs).total;
 }
 
-// BiCGStab on instances of at least 2^23 cells runs as per-phase kernels in a CUDA graph even in
-// the persistent mode: at that size the separate kernels, each at its own full occupancy, move
-// the iteration's bytes faster than the cooperative kernel (measured on one B200 with float32
-// iterations: 0.52 against 0.44 of HBM on 256^3, 0.57 against 0.52 on 4096^2); CG keeps the
-// persistent kernel (0.62 against 0.53).
-static bool bicgPrefersGraph(const phb_domain *dom, int kind) {
-	return kind == 1 && dom->ninst > 0 && dom->ncells / dom->ninst >= (int64_t(1) << 23);
+// BiCGStab of one float32 or of two right-hand sides on instances of at least 2^23 cells runs as per-phase
+// kernels in a CUDA graph even in the persistent mode. On rows of four cells the persistent kernel is the faster one
+// at every size (4096^2 float32, two right-hand sides 666 against 808 us an iteration, one 399 against 492), but on
+// odd rows, which it takes a cell at a time, it loses there (4001 x 4003: 1299 against 979 and 717 against
+// 571; 254 x 253 x 250, one: 964 against 730), and the row length is not known to the host. With three
+// right-hand sides and with one in float64 it is as fast or faster on all of them (256^3 float32 three 1095 against
+// 1312, 251 x 253 x 249 1861 against 2073, 4001 x 4003 float64 one 886 against 893).
+static bool bicgPrefersGraph(const phb_domain *dom, int kind, bool f32, int nrhs) {
+	return kind == 1 && (nrhs == 2 || (nrhs == 1 && f32)) && dom->ninst > 0 && dom->ncells / dom->ninst >= (int64_t(1) << 23);
 }
 
 extern "C" int phb_solve_run(const phb_domain *dom, const phb_solve *s_in, phb_stream stream) {
 	phb_solve sAdj;
 	const phb_solve *s = s_in;
-	if (s_in && dom && s_in->use_graph == 2 && bicgPrefersGraph(dom, s_in->kind)) {
+	if (s_in && dom && s_in->use_graph == 2 && bicgPrefersGraph(dom, s_in->kind, s_in->vec_dtype == PHB_F32, s_in->nrhs)) {
 		sAdj = *s_in;
 		sAdj.use_graph = 1;
 		s = &sAdj;
@@ -1112,7 +1114,7 @@ static int emitRefine(const phb_domain *dom, const phb_refine *rf, cudaStream_t 
 	// persistent inner solves (every launch visible to a kernel profiler); 0: host loops
 	const bool graph = rf->use_graph == 1 || rf->use_graph == 2;
 	in.use_graph = rf->use_graph >= 2 ? 2 : (graph ? 1 : 0);
-	if (rf->use_graph == 2 && bicgPrefersGraph(dom, rf->kind)) in.use_graph = 1; // nested graph loop
+	if (rf->use_graph == 2 && bicgPrefersGraph(dom, rf->kind, true, K)) in.use_graph = 1; // nested graph loop
 	in.check_every = 8;
 	cudaGraphConditionalHandle outerHandle{};
 	if (graph) {

@@ -8,7 +8,7 @@ import torch
 import phipict_b200 as pb
 from phipict_b200 import _C
 from phipict_b200.solvers import BICGSTAB, CG, solver_for
-from cases import duct_3d, hartmann_2d, rotated_pair_2d, seeded_state
+from cases import duct_3d, hartmann_2d, periodic_box_3d, rotated_pair_2d, rotated_pair_3d, seeded_state
 
 pytestmark = pytest.mark.gpu
 
@@ -19,6 +19,10 @@ CASES = {
     "wide_3d": lambda **k: duct_3d(48, 40, 20, 2, **k),        # 76 tiles: the grid kernel
     "wide_odd_3d": lambda **k: duct_3d(37, 25, 23, 2, **k),
     "rotated_2d": lambda **k: rotated_pair_2d(16, **k),
+    "rotated_3d": lambda **k: rotated_pair_3d(**k),
+    "rotated_swapped_3d": lambda **k: rotated_pair_3d((8, 12, 8), 16, swapped=True, **k),  # rows of four beside it
+    "rotated_wide_3d": lambda **k: rotated_pair_3d((32, 24, 28), 36, **k),                 # the grid kernel
+    "periodic_3d": lambda **k: periodic_box_3d(32, 36, 40, **k),
     "one_tile": lambda **k: hartmann_2d(32, 24, **k),
     "two_tiles": lambda **k: hartmann_2d(64, 32, **k),
     "three_tiles_odd": lambda **k: hartmann_2d(51, 53, **k),
@@ -167,3 +171,32 @@ def test_a_batch_of_more_clusters_than_fit_at_a_time(cuda):
     (x0, t0), (x1, t1) = run(0), run(3)
     assert torch.equal(x0, x1)
     assert t0 < 1.5 * t1, (t0, t1)
+
+
+# Tiles per worker group at one group per SM: more than 8 (the sums of a phase are flushed in its middle,
+# forwards and backwards), more than 16 (the tile list goes on in global memory), and more than 256 tiles
+# of one instance (several rounds of loads in its sums)
+LONG = {
+    "rows_of_four_2d": lambda **k: hartmann_2d(1600, 1600, **k),  # 2500 tiles
+    "odd_2d": lambda **k: hartmann_2d(1601, 1597, **k),           # 2497 tiles
+    "rows_of_four_3d": lambda **k: duct_3d(128, 104, 100, 1, **k),  # 1300 tiles
+    "odd_3d": lambda **k: duct_3d(137, 139, 133, 1, **k),          # 2474 tiles
+    "large_3d": lambda **k: duct_3d(256, 184, 180, 1, **k),        # 8280 tiles, past 2^23 cells
+}
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64], ids=["f32", "f64"])
+@pytest.mark.parametrize("case", list(LONG))
+def test_long_tile_lists_match_per_phase_kernels(cuda, case, dtype):
+    dom = LONG[case](dtype=dtype)
+    seeded_state(dom, 5, scale=0.2)
+    dom.PrepareSolve()
+    _assemble(dom, 5)
+    assert dom.desc().ntiles > 8 * 148
+    d = dom.getSpatialDims()
+    for kind, A, nrhs, its in ((CG, dom._P_st, 1, 7), (BICGSTAB, dom._C_st, 1, 4), (BICGSTAB, dom._C_st, d, 4)):
+        b = _rhs(dom, dom.numCells(), nrhs, 7)
+        ref = _solve(dom, kind, nrhs, A, b, 1e-30, its, 1)
+        assert all(i.isFiniteResidual for i in ref[1])
+        for ctas in (0, 1):
+            assert _same(_solve(dom, kind, nrhs, A, b, 1e-30, its, 2, ctas=ctas), ref), (kind, nrhs, ctas)
