@@ -563,14 +563,16 @@ __global__ void __launch_bounds__(PHB_TILE *PCG_GROUPS, 1) kPcg(const __grid_con
 		const int row = l / B.nx, z = D > 2 ? row / B.ny : 0;
 		f(B.off + l, l - row * B.nx, row - z * B.ny, z);
 	};
-	// cells 256 apart (loads of a warp stay contiguous whatever the row length), two at a time
-	auto cells = [&](const BlockTab &B, int l0, auto f) {
+	// cells 256 apart (loads of a warp stay contiguous whatever the row length), two at a time; the one cell
+	// per thread of a quarter tile by itself
+	auto cellsOf = [&](auto width, const BlockTab &B, int l0, auto f) {
+		constexpr int W = decltype(width)::value;
 		const int end = min(B.cells(), l0 + cells0);
-		for (int l = l0 + wk.lt; l < end; l += 2 * PHB_TILE) {
-			int g[2], x[2], y[2], z[2];
-			const int n = l + PHB_TILE < end ? 2 : 1;
+		for (int l = l0 + wk.lt; l < end; l += W * PHB_TILE) {
+			int g[W], x[W], y[W], z[W];
+			const int n = W > 1 && l + PHB_TILE < end ? 2 : 1;
 #pragma unroll
-			for (int j = 0; j < 2; ++j) {
+			for (int j = 0; j < W; ++j) {
 				const int lj = j < n ? l + j * PHB_TILE : l;
 				const int row = lj / B.nx;
 				z[j] = D > 2 ? row / B.ny : 0;
@@ -578,8 +580,12 @@ __global__ void __launch_bounds__(PHB_TILE *PCG_GROUPS, 1) kPcg(const __grid_con
 				y[j] = row - z[j] * B.ny;
 				g[j] = B.off + lj;
 			}
-			f(n, g, x, y, z);
+			f(width, n, g, x, y, z);
 		}
+	};
+	auto cells = [&](const BlockTab &B, int l0, auto f) {
+		if (quarter) cellsOf(Count<1>{}, B, l0, f);
+		else cellsOf(Count<2>{}, B, l0, f);
 	};
 	float *rIn = a.r0, *rOut = a.r1, *pIn = a.p0, *pOut = a.p1;
 	// r = b - A x, (r, r), (b, b)
@@ -602,15 +608,16 @@ __global__ void __launch_bounds__(PHB_TILE *PCG_GROUPS, 1) kPcg(const __grid_con
 				st4f(rIn + g, yv);
 			});
 		} else {
-			cells(B, l0, [&](int n, const int (&g)[2], const int (&x)[2], const int (&y)[2], const int (&z)[2]) {
-				float fc, rv[2], bv[2];
+			cells(B, l0, [&](auto width, int n, const auto &g, const auto &x, const auto &y, const auto &z) {
+				constexpr int W = decltype(width)::value;
+				float fc, rv[W], bv[W];
 #pragma unroll
-				for (int j = 0; j < 2; ++j) {
+				for (int j = 0; j < W; ++j) {
 					bv[j] = a.b[g[j]];
 					rv[j] = bv[j] - pcgCellApply<D>(B, g[j], x[j], y[j], z[j], N, a.A, fx, fc);
 				}
 #pragma unroll
-				for (int j = 0; j < 2; ++j)
+				for (int j = 0; j < W; ++j)
 					if (j < n) {
 						acc[0] = fma(double(rv[j]), double(rv[j]), acc[0]);
 						acc[1] = fma(double(bv[j]), double(bv[j]), acc[1]);
@@ -717,15 +724,16 @@ __global__ void __launch_bounds__(PHB_TILE *PCG_GROUPS, 1) kPcg(const __grid_con
 						st4f(zz + g, out);
 					});
 				} else {
-					cells(B, l0, [&](int n, const int (&g)[2], const int (&x)[2], const int (&y)[2], const int (&z)[2]) {
-						float out[2], rv[2];
+					cells(B, l0, [&](auto width, int n, const auto &g, const auto &x, const auto &y, const auto &z) {
+						constexpr int W = decltype(width)::value;
+						float out[W], rv[W];
 #pragma unroll
-						for (int j = 0; j < 2; ++j) {
+						for (int j = 0; j < W; ++j) {
 							rv[j] = rIn[g[j]];
 							out[j] = pcgProlongCell<D>(B, cblk[b], g[j], x[j], y[j], z[j], N, a.A, a.mg.wd[0], rv[j], zz[g[j]], e);
 						}
 #pragma unroll
-						for (int j = 0; j < 2; ++j)
+						for (int j = 0; j < W; ++j)
 							if (j < n) {
 								acc[0] = fma(double(rv[j]), double(out[j]), acc[0]);
 								zz[g[j]] = out[j];
@@ -754,12 +762,13 @@ __global__ void __launch_bounds__(PHB_TILE *PCG_GROUPS, 1) kPcg(const __grid_con
 					st4f(a.q + g, yv);
 				});
 			} else {
-				cells(B, l0, [&](int n, const int (&g)[2], const int (&x)[2], const int (&y)[2], const int (&z)[2]) {
-					float yv[2], fc[2];
+				cells(B, l0, [&](auto width, int n, const auto &g, const auto &x, const auto &y, const auto &z) {
+					constexpr int W = decltype(width)::value;
+					float yv[W], fc[W];
 #pragma unroll
-					for (int j = 0; j < 2; ++j) yv[j] = pcgCellApply<D>(B, g[j], x[j], y[j], z[j], N, a.A, fd, fc[j]);
+					for (int j = 0; j < W; ++j) yv[j] = pcgCellApply<D>(B, g[j], x[j], y[j], z[j], N, a.A, fd, fc[j]);
 #pragma unroll
-					for (int j = 0; j < 2; ++j)
+					for (int j = 0; j < W; ++j)
 						if (j < n) {
 							acc[0] = fma(double(fc[j]), double(yv[j]), acc[0]);
 							pOut[g[j]] = fc[j];
