@@ -280,7 +280,8 @@ typedef struct phb_solve {
 	int32_t use_graph;    /* 2 (or 3): persistent cooperative kernel; 1: conditional-WHILE CUDA graph; 0: host loop */
 	int32_t check_every;  /* host loop only: iterations between completion checks */
 	phb_tolerance tol;
-	const void *A;        /* stencil [2d+1][ncells] */
+	const void *A;        /* stencil [2d+1][ncells], 0 in the slots across prescribed faces (as every
+	                         matrix kernel here writes): the products multiply them */
 	const void *b;        /* [inst][nrhs][cells] */
 	void *x;              /* in: initial guess, out: solution */
 	void *work;           /* >= phb_solve_work_bytes() bytes, 256-byte aligned */

@@ -1016,7 +1016,8 @@ extern "C" int phb_solve_results(const phb_domain *dom, const phb_solve *s, phb_
 extern "C" int phb_stencil_apply(const phb_domain *dom, const double *A, const double *X, double *Y, int32_t nvec,
 		int64_t stride, phb_stream stream) {
 	if (!dom || !A || !X || !Y) return setError(PHB_ERR_ARG, "phb_stencil_apply: null argument");
-	// the quad loads of a row take 16-byte vector loads at cells that are multiples of four
+	// the layout that the header asks of callers, wide enough for vector loads of rows of four (the kernel takes
+	// a cell at a time)
 	if (nvec < 1 || stride < dom->ncells || (stride & 3) != 0)
 		return setError(PHB_ERR_ARG, "phb_stencil_apply: nvec < 1, stride < ncells or stride not a multiple of 4");
 	if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 31)

@@ -396,8 +396,6 @@ __device__ __forceinline__ void pcgQuadApply(const BlockTab &B, int g, int x, in
 		const F &f, float (&yv)[4], float (&fc)[4]) {
 	int o[2 * D];
 	const unsigned int has = tabNeighbors<D, 4>(B, g, x, y, z, o);
-	// the +x neighbour across a block face is that of the row's last cell
-	if (x + 4 == B.nx && (has & 2)) o[1] = tabMap(B.map[1], x + 3, y, z);
 	float a[4], v[2 * D - 2][4];
 	f.at4(g, 4, true, fc);
 	float w = f.at(o[0]), e = f.at(o[1]);

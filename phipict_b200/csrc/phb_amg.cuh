@@ -549,15 +549,15 @@ __device__ __forceinline__ double amgProlongQuad(const AmgView<D> &mg, int l, in
 // inverse, or the folded cycle below it), one warp per row; rows are dealt out to warps
 // `warp`, `warp + nwarps`, ...
 template <int D>
-__device__ __forceinline__ void amgCoarseRows(const AmgView<D> &mg, int warp, int nwarps, int row0 = 0, int row1 = -1) {
+__device__ __forceinline__ void amgCoarseRows(const AmgView<D> &mg, int warp, int nwarps) {
 	const int L = mg.nlevels - 1;
 	const Dom<float, D> &cd = mg.lv[L];
 	const int lane = threadIdx.x & 31;
 	const int cn = mg.cn;
 	const float *b = mg.b[L];
 	float *x = mg.x[L];
-	const int rows = row1 < 0 ? cd.ninst * cn : row1;
-	for (int row = row0 + warp; row < rows; row += nwarps) {
+	const int rows = cd.ninst * cn;
+	for (int row = warp; row < rows; row += nwarps) {
 		const int inst = row / cn, r = row - inst * cn;
 		const int off = __ldg(cd.insts + inst * PHB_IREC + I_CELLOFF);
 		const int n = min(cn, __ldg(cd.insts + inst * PHB_IREC + I_NCELLS));
