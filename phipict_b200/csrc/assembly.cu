@@ -20,11 +20,12 @@ namespace phb {
 
 // CTAs per SM that the register budget of the branch-free kernels allows: a 3D float64 cell has 55
 // loads in flight (128 registers; at three CTAs the matrix on 192^3 took 484 instead of 351 us), the
-// others fit 85 (1999x1501 float32: 69 instead of 83 us). On large grids some run better
-// with more warps and fewer loads in flight, or the other way round (4096^2, CTAs per SM; us): HbyA float32
-// 386 at 3, 277 at 5, 302 at 6; velocity correction float32 194 at 4, 135 at 6; pressure matrix float64 324 at 3, 306 at 5;
-// divergence float64 344 at 3, 284 at 4; u x e_b with its right-hand side float64 411 at 3, 344 at 4; potential
-// right-hand side float64 335 at 3, 273 at 5, float32 on 192^3 222 at 3, 174 at 2.
+// others fit 85 (1999x1501 float32: 69 instead of 83 us). On large grids some run better with more warps and
+// fewer loads in flight, or the other way round (us at CTAs per SM, 4096^2 unless said otherwise):
+// HbyA float32 386 at 3, 277 at 5, 302 at 6; velocity correction float32 194 at 4, 135 at 6; pressure matrix float64
+// 324 at 3, 316 at 4, 306 at 5, but with its float32 copy 365, 367 and 454; divergence float64 344 at 3, 284 at 4;
+// u x e_b with its right-hand side float64 411 at 3, 344 at 4; potential right-hand side float64 335 at 3, 273 at 5,
+// float32 on 192^3 222 at 3, 174 at 2.
 enum AsmKernel { K_ADV_MATRIX, K_ADV_RHS, K_P_MATRIX, K_HBYA, K_DIVERGENCE, K_CORRECT, K_UXB, K_EPOT };
 template <AsmKernel K, typename S, int D, int PARTS>
 constexpr int asmCtas() {
@@ -32,8 +33,8 @@ constexpr int asmCtas() {
 	if (PARTS == 1 && D == 2) {
 		if (K == K_HBYA && !f64) return 5;
 		if (K == K_CORRECT && !f64) return 6;
-		if ((K == K_P_MATRIX || K == K_EPOT) && f64) return 5;
-		if ((K == K_DIVERGENCE || K == K_UXB) && f64) return 4;
+		if (K == K_EPOT && f64) return 5;
+		if ((K == K_P_MATRIX || K == K_DIVERGENCE || K == K_UXB) && f64) return 4;
 	}
 	if (PARTS == 1 && D == 3 && K == K_EPOT) return 2;
 	if (K == K_ADV_RHS || K == K_CORRECT) return 4;
@@ -693,7 +694,7 @@ __global__ void __launch_bounds__(PHB_TILE, sizeof(S) == 8 ? 2 : 3) kPressureRhs
 }
 
 // HbyA of the central scheme, one cell at a time with all its loads in flight together: the row form
-// above resolves the faces of the quads that touch one (192^3 float64: 585 us in that form, 408 here).
+// above resolves the faces of the quads that touch one (192^3 float64: 569 us in that form, 371 here).
 template <typename S, int D, int PARTS>
 __global__ void __launch_bounds__(PHB_TILE, (asmCtas<K_HBYA, S, D, PARTS>())) kPressureRhsCentral(Dom<S, D> dom, int run, const S *__restrict__ C, const S *__restrict__ Adiag,
 		const S *__restrict__ u, const S *__restrict__ ustar, const S *__restrict__ src, int srcMode, S *__restrict__ hbya) {
