@@ -155,9 +155,9 @@ def algorithmic_pcg_bytes(dims: int, levels: list[int], dense_doubles: int = 0) 
 
 
 # DRAM bytes per preconditioned CG iteration on the duct workload, from a full ncu capture of
-# one persistent launch (the first inner solve of the timed step: 26.11 MB read + 0.57 MB
-# written in a 24-iteration solve): the working set is L2-resident
-PCG_DRAM_BYTES_PER_ITERATION_DUCT3D = (26.11e6 + 0.57e6) / 24
+# one launch of kPcg (profiles/kPcg_duct3d_full.md: 26.7 MB read + 0.4 MB written in a solve of
+# about 24 iterations): the working set is L2-resident
+PCG_DRAM_BYTES_PER_ITERATION_DUCT3D = (26.7e6 + 0.4e6) / 24
 
 
 class ClockSampler:
