@@ -19,9 +19,9 @@
 // are formed before its loads, and the loads are issued without a branch between them: a face
 // resolved by a branch of its own costs its own round trip to L2, which made most of an iteration
 // of the form before this one. Microseconds per iteration, before and after (B200):
-//   3 blocks 64x48x48 (442,368 cells, rows of four)          67 -> 42
-//   2 blocks 37x45x41 (136,530 cells, odd rows)               72 -> 39
-//   128^3 (2.1 M cells)                                      213 -> 99
+//   3 blocks 64x48x48 (442,368 cells, rows of four)          67 -> 40
+//   2 blocks 37x45x41 (136,530 cells, odd rows)               72 -> 37
+//   128^3 (2.1 M cells)                                      213 -> 98
 //   64 2D instances of 32^2 to 256^2 (1.2 M cells)           170 -> 77
 //   6 3D instances of 32^3 to 112^3 (3.6 M cells, odd rows)  430 -> 226
 #include "phb_krylov.cuh"
